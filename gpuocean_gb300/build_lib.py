@@ -40,6 +40,7 @@ EXTRA = {"noise.cu": ["-use_fast_math"],
          "drift.cu": ["-fmad=false"],
          "cdklm_step.cu": ["-fmad=false"],
          "ensemble.cu": ["-fmad=false"],
+         "ensemble_march.cu": ["-fmad=false"],
          **{f"ensemble_shape_{tx}x{ty}.cu": ["-fmad=false"]
             for tx, ty in ((32, 16), (32, 8), (16, 16), (64, 8), (32, 24))}}
 

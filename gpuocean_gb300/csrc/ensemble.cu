@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(256) ensemble_dt_final_kernel(const float* __r
 static void free_ensemble(Ensemble* e) {
     cudaFree(e->d_members);
     cudaFree(e->d_tiles);
+    cudaFree(e->d_march);
     cudaFree(e->d_dt);
     cudaFree(e->d_nsub);
     cudaFree(e->d_dt_items);
@@ -165,7 +166,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // loads.  The depth (and Coriolis) boxes follow the same rules.
 static int build_tma_maps(Ensemble* e) {
     const int n = e->n_members;
-    std::vector<CUtensorMap> maps((size_t)kNumEnsembleShapes * n * kTmaMapsPerMember);
+    std::vector<CUtensorMap> maps((size_t)kMarchShape * n * kTmaMapsPerMember);
     std::vector<const float*> base(n, nullptr);
     std::vector<int> aux(n, 0);
     const PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
@@ -190,7 +191,7 @@ static int build_tma_maps(Ensemble* e) {
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
         };
-        for (int sh = 0; ok && sh < kNumEnsembleShapes; ++sh) {
+        for (int sh = 0; ok && sh < kMarchShape; ++sh) {
             CUtensorMap* mm = &maps[((size_t)sh * n + m) * kTmaMapsPerMember];
             const cuuint32_t bx = (cuuint32_t)kEnsembleShapes[sh].tx + 8, by = (cuuint32_t)kEnsembleShapes[sh].ty + 8;
             for (int set = 0; ok && set < 2; ++set)
@@ -246,7 +247,11 @@ const int* ensemble_device_nsub(void* ensemble) { return static_cast<Ensemble*>(
 const int* ensemble_device_noise_steps(void* ensemble) { return static_cast<Ensemble*>(ensemble)->d_nsub_noise; }
 
 static int shape_configure(const Ensemble* e, int* grid) {
-    switch (e->shape) {
+    if (e->shape == kMarchShape && e->can_march) {
+        const int rc = ensemble_march_configure(e, grid);
+        if (rc) return rc;
+    }
+    switch (e->tile_shape()) {
         case 0: return ensemble_configure_shape<32, 16>(e, grid);
         case 1: return ensemble_configure_shape<32, 8>(e, grid);
         case 2: return ensemble_configure_shape<16, 16>(e, grid);
@@ -257,7 +262,8 @@ static int shape_configure(const Ensemble* e, int* grid) {
 }
 
 static int shape_launch(Ensemble* e, int k, cudaStream_t st, const FusedNoise* fn) {
-    switch (e->shape) {
+    if (e->shape == kMarchShape && e->can_march && !(fn && fn->noise)) return ensemble_march_launch(e, k, st, fn);
+    switch (e->tile_shape()) {
         case 0: return ensemble_launch_shape<32, 16>(e, k, st, fn);
         case 1: return ensemble_launch_shape<32, 8>(e, k, st, fn);
         case 2: return ensemble_launch_shape<16, 16>(e, k, st, fn);
@@ -283,8 +289,49 @@ static bool host_tile_on_border(const GocCdklmParams& p, int tx, int ty, int i, 
     return x0 < 2 || y0 < 2 || x0 + tx + 8 > p.nx + 2 || y0 + ty + 8 > p.ny + 2;
 }
 
+// Units of kMarchShape's rows per run of the marching kernel: a run costs its
+// rows plus about four (the rows below and above it that it computes again),
+// so runs are as long as leaves about four per resident warp to even out the
+// end of the launch.
+static int build_march(Ensemble* e) {
+    cudaFree(e->d_march);
+    e->d_march = nullptr;
+    e->n_march = 0;
+    int grid = 0;
+    const int rc = ensemble_march_configure(e, &grid);
+    if (rc) return rc;
+    const TileShape sh = kEnsembleShapes[kMarchShape];
+    long long units = 0;
+    for (const GocMemberDesc& d : e->host)
+        units += (long long)((d.p.nx + sh.tx - 1) / sh.tx) * ((d.p.ny + sh.ty - 1) / sh.ty);
+    const int most = (int)std::min(16LL, std::max(1LL, units / (4LL * grid)));
+    std::vector<int4> runs;
+    for (int m = 0; m < e->n_members; ++m) {
+        const GocCdklmParams& p = e->host[m].p;
+        const int strips = (p.nx + sh.tx - 1) / sh.tx, len = (p.ny + sh.ty - 1) / sh.ty;
+        const int n = (len + most - 1) / most;
+        for (int i = 0; i < strips; ++i)
+            for (int r = 0, j = 0; r < n; ++r) {
+                const int w = len / n + (r < len % n ? 1 : 0);
+                runs.push_back(make_int4(m, i, j, w));
+                j += w;
+            }
+    }
+    std::stable_sort(runs.begin(), runs.end(), [](const int4& a, const int4& b) { return a.w > b.w; });
+    cudaError_t err = cudaMalloc(&e->d_march, sizeof(int4) * runs.size());
+    if (err == cudaSuccess)
+        err = cudaMemcpy(e->d_march, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice);
+    if (err != cudaSuccess) return set_error(GOC_ERR_CUDA, "ensemble march queue: %s", cudaGetErrorString(err));
+    e->n_march = (int)runs.size();
+    return GOC_OK;
+}
+
 static int build_tiles(Ensemble* e) {
-    const TileShape sh = kEnsembleShapes[e->shape];
+    const TileShape sh = kEnsembleShapes[e->tile_shape()], count = kEnsembleShapes[e->shape];
+    if (e->shape == kMarchShape && e->can_march) {
+        const int rc = build_march(e);
+        if (rc) return rc;
+    }
     std::vector<int4> inner, border;
     int n_tiles = 0;
     for (int m = 0; m < e->n_members; ++m) {
@@ -303,7 +350,7 @@ static int build_tiles(Ensemble* e) {
                     j += n;
                 }
             }
-        n_tiles += tx * ty;
+        n_tiles += ((p.nx + count.tx - 1) / count.tx) * ((p.ny + count.ty - 1) / count.ty);
     }
     auto longest_first = [](const int4& a, const int4& b) { return a.w > b.w; };
     std::stable_sort(inner.begin(), inner.end(), longest_first);
@@ -337,6 +384,8 @@ extern "C" int goc_ensemble_create(const GocMemberDesc* members, int n_members, 
     e->host.assign(members, members + n_members);
     std::vector<int4> dt_items;
     std::vector<int2> ranges;
+    bool can_march = true;
+    int with_table = 0;
     for (int m = 0; m < n_members; ++m) {
         const GocMemberDesc& d = members[m];
         char who[64];
@@ -357,12 +406,17 @@ extern "C" int goc_ensemble_create(const GocMemberDesc* members, int n_members, 
         e->const_f = e->const_f && d.p.coriolis_nx == 1 && d.p.coriolis_ny == 1;
         e->simple = e->simple && d.p.wind_x_nx == 1 && d.p.wind_x_ny == 1 && d.p.wind_y_nx == 1 &&
                     d.p.wind_y_ny == 1 && d.p.atm_p_nx == 1 && d.p.atm_p_ny == 1;
+        // the marching kernel takes uniform forcing, one Coriolis value or a
+        // table per cell, and grids on which a wall's mirror images exist
+        can_march = can_march && d.p.nx >= 2 && d.p.ny >= 2;
+        with_table += d.p.coriolis_cell != nullptr;
         const int bx = (d.p.nx + kDtBX - 1) / kDtBX, by = (d.p.ny + kDtBY - 1) / kDtBY;
         ranges.push_back(make_int2((int)dt_items.size(), bx * by));
         for (int j = 0; j < by; ++j)
             for (int i = 0; i < bx; ++i) dt_items.push_back(make_int4(m, i, j, (int)dt_items.size()));
     }
     e->n_dt_items = (int)dt_items.size();
+    e->can_march = can_march && e->simple && (e->const_f || with_table == n_members);
     // shared scalar parameters: every member's parameters equal member 0's
     // once the texture pointers are set aside (those stay per member)
     auto scalars = [](GocCdklmParams q) {
@@ -631,6 +685,13 @@ extern "C" int goc_ensemble_set_tile_shape(void* ensemble, int index) {
 extern "C" int goc_ensemble_get_tile_shape(void* ensemble, int* index) {
     if (!ensemble || !index) return set_error(GOC_ERR_ARG, "goc_ensemble_get_tile_shape: null argument");
     *index = static_cast<Ensemble*>(ensemble)->shape;
+    return GOC_OK;
+}
+
+extern "C" int goc_ensemble_marches(void* ensemble, int* marches) {
+    if (!ensemble || !marches) return set_error(GOC_ERR_ARG, "goc_ensemble_marches: null argument");
+    const Ensemble* e = static_cast<Ensemble*>(ensemble);
+    *marches = e->shape == kMarchShape && e->can_march;
     return GOC_OK;
 }
 

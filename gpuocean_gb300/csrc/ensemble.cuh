@@ -16,8 +16,11 @@ namespace goc {
 // Output tile shapes (cells) the engine can run; the autotuner picks one per
 // ensemble.  Index 0 is the default.
 struct TileShape { int tx, ty; };
-constexpr TileShape kEnsembleShapes[] = {{32, 16}, {32, 8}, {16, 16}, {64, 8}, {32, 24}};
+// The last one stands for the marching kernel (cdklm_march.cuh): strips of 56
+// columns, runs counted in units of 8 rows.
+constexpr TileShape kEnsembleShapes[] = {{32, 16}, {32, 8}, {16, 16}, {64, 8}, {32, 24}, {56, 8}};
 constexpr int kNumEnsembleShapes = sizeof(kEnsembleShapes) / sizeof(kEnsembleShapes[0]);
+constexpr int kMarchShape = kNumEnsembleShapes - 1;
 constexpr int kTmaMapsPerMember = 16;
 
 // CTAs per SM the shared memory of a shape allows (at most 3), used as the
@@ -44,7 +47,7 @@ struct Ensemble {
     std::vector<GocMemberDesc> host;      // descriptors as created (set 0 current)
     GocMemberDesc* d_members = nullptr;   // device copy, buffers swapped on device
     int4* d_tiles = nullptr;              // runs (member, tile_x, first tile_y, tiles)
-    // [shape][member][kTmaMapsPerMember] TMA maps: eta, hu, hv main boxes of
+    // [tile shape][member][kTmaMapsPerMember] TMA maps: eta, hu, hv main boxes of
     // buffer sets 0 and 1, their east boxes, then the cell-mean depth and the
     // Coriolis table (main, east)
     CUtensorMap* d_tmaps = nullptr;
@@ -93,6 +96,13 @@ struct Ensemble {
     std::vector<int> nsub_noise_host;
     int* d_nsub_noise = nullptr;
     int shape = 0;                        // index into kEnsembleShapes
+    // The marching kernel's queue (shape kMarchShape) and whether that kernel
+    // steps every member; launches with fused model error, and ensembles it
+    // does not take, run the tile kernel of tile_shape (then shape 0).
+    int4* d_march = nullptr;
+    int n_march = 0;
+    bool can_march = false;
+    int tile_shape() const { return shape == kMarchShape ? 0 : shape; }
 };
 
 constexpr int kDriftChunk = 256;
@@ -102,19 +112,15 @@ __device__ __forceinline__ DriftGrid member_drift_grid(const GocMemberDesc& d, i
                      d.Hm, d.Hm_pitch / 4, d.p.bc_north == 2, d.p.bc_east == 2};
 }
 
-// Advect one chunk of a member's drifters with the state of buffer set `set`
-// (or, with `copy`, the unperturbed copy of that state: the drift of the
-// last step of a block whose model error was fused into that step).
+// Advect one chunk of a member's drifters with the state of buffer set
+// `set`; thread t of the nt that share the chunk.
 __device__ __forceinline__ void drift_chunk(const GocMemberDesc& d, float* pos, int first, int count, int set,
-                                           float dt, float sensitivity, float* const* copy = nullptr) {
+                                           float dt, float sensitivity, int t, int nt) {
     const DriftGrid g = member_drift_grid(d, set);
-    for (int q = threadIdx.x; q < count; q += blockDim.x) {
+    for (int q = t; q < count; q += nt) {
         float* p = pos + 2 * (size_t)(first + q);
         float px = p[0], py = p[1];
-        if (copy)
-            drift_one_with(g, CopyVelocity{g, copy[0], copy[1], copy[2]}, nullptr, dt, sensitivity, px, py);
-        else
-            drift_one(g, nullptr, dt, sensitivity, px, py);
+        drift_one(g, nullptr, dt, sensitivity, px, py);
         p[0] = px;
         p[1] = py;
     }
@@ -189,7 +195,7 @@ ensemble_rk2_kernel(const GocCdklmParams pu, const StepConst ku, const GocMember
             // (ensemble_end_drift_kernel) that keeps this kernel's code small
             if (spare && k == ns && k == __ldg(noise_steps + c.x) && spare[3 * c.x]) continue;
             drift_chunk(members[c.x], drift_pos[c.x], c.y, c.z, k & 1,
-                        __ldg(dt_table + (size_t)c.x * max_sub + (k - 1)), sensitivity);
+                        __ldg(dt_table + (size_t)c.x * max_sub + (k - 1)), sensitivity, threadIdx.x, blockDim.x);
             continue;
         }
         // a run of t.w consecutive tiles of the column strip t.y, from tile row t.z
@@ -328,7 +334,7 @@ int launch_ensemble(Ensemble* e, int k, cudaStream_t st, const FusedNoise* fn) {
     kern<<<grid, kNT, smem, st>>>(e->pu, e->ku, e->d_members, e->d_tiles, e->n_runs, e->d_dt, e->d_nsub,
                                   e->max_substeps, k, e->d_drift_pos, e->d_step_chunks, e->n_step_chunks,
                                   e->drift_sensitivity,
-                                  e->d_tmaps + (size_t)e->shape * e->n_members * kTmaMapsPerMember,
+                                  e->d_tmaps + (size_t)e->tile_shape() * e->n_members * kTmaMapsPerMember,
                                   e->d_tma_base, e->d_tma_aux, e->d_tma_err, e->d_tma_tiles, fn ? fn->noise : nullptr,
                                   fn ? fn->spare : nullptr, fn ? fn->mode : 0, e->d_nsub_noise, e->d_queue);
     count_launch();
@@ -378,6 +384,10 @@ int ensemble_launch_shape(Ensemble* e, int k, cudaStream_t st, const FusedNoise*
     if (e->simple) return launch_variant<TX, TY, false, true>(e, k, st, fn);
     return launch_variant<TX, TY, false, false>(e, k, st, fn);
 }
+
+// The marching kernel (ensemble_march.cu).
+int ensemble_march_configure(const Ensemble* e, int* grid);
+int ensemble_march_launch(Ensemble* e, int k, cudaStream_t st, const FusedNoise* fn);
 
 #define GOC_ENSEMBLE_SHAPE_EXTERN(TX, TY)                                           \
     extern template int ensemble_configure_shape<TX, TY>(const Ensemble*, int*);     \

@@ -376,6 +376,12 @@ class BatchedEnsemble:
     def tile_shape(self):
         return self.tile_shapes()[self._shape_index]
 
+    def _marches(self):
+        """Whether the steps run the marching kernel."""
+        out = ctypes.c_int()
+        _lib.call("goc_ensemble_marches", self._handle, ctypes.byref(out))
+        return bool(out.value)
+
     def set_tile_shape(self, index):
         _lib.call("goc_ensemble_set_tile_shape", self._handle, int(index))
         self._shape_index = int(index)
@@ -597,13 +603,14 @@ class BatchedEnsemble:
 
     def _launch_block(self, nsub, noise=None, n=None):
         """noise: None, "block" (once after the block) or "step" (after every
-        RK2 step of each member, before its drifters move).  SOAR model error
-        is fused into the step launches: the coarse fields are computed
-        before the first step that perturbs, and each member's perturbation
-        is added to the state the step writes.  KL model error runs as its
-        own launches after the steps.  n: the members' step counts."""
+        RK2 step of each member, before its drifters move).  With a tile
+        kernel, SOAR model error is fused into the step launches: the coarse
+        fields are computed before the first step that perturbs, and each
+        member's perturbation is added to the state the step writes.  With
+        the marching kernel, and for KL model error, it runs as its own
+        launches after the steps.  n: the members' step counts."""
         before = _lib.load().goc_kernel_launch_count()
-        fused = noise is not None and self._noise_kind == "soar"
+        fused = noise is not None and self._noise_kind == "soar" and not self._marches()
         first = -1
         if fused:
             _lib.call("goc_ensemble_set_block_noise", self._handle, self._noise, 0 if noise == "block" else 1)
@@ -620,7 +627,14 @@ class BatchedEnsemble:
             if fused:
                 _lib.call("goc_ensemble_set_block_noise", self._handle, None, -1)
         if noise == "block" and not fused:
-            self._noise_launch(-2)   # the members that take model error in this block
+            # the members that take model error in this block; SOAR draws new
+            # normals for every member, as ahead of a fused step
+            if self._noise_kind == "soar":
+                if self._rng_seed is not None:
+                    _lib.call("goc_noise_batch_generate", self._noise, self._handle, -1, self.stream.handle)
+                self._noise_launch(-2, update_random_field=False)
+            else:
+                self._noise_launch(-2)
         return _lib.load().goc_kernel_launch_count() - before
 
     def step(self, t_end, apply_stochastic_term=False, noise_cadence="block", members=None):

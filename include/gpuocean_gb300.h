@@ -523,6 +523,15 @@ int goc_ensemble_tile_shape(int index, int* tx, int* ty);
 int goc_ensemble_set_tile_shape(void* ensemble, int index);
 int goc_ensemble_get_tile_shape(void* ensemble, int* index);
 
+/* Whether the ensemble's steps run the marching kernel: its tile shape (the
+ * last one) is set and the kernel takes every member.  Launches with fused
+ * model error (goc_ensemble_set_block_noise) run a tile kernel all the same:
+ * with a marching ensemble, perturb after goc_ensemble_end_block instead
+ * (goc_noise_batch_perturb with substep -2, or substep k after step k); the
+ * states are the same bits.
+ */
+int goc_ensemble_marches(void* ensemble, int* marches);
+
 /* Close a block of `n_launched` substeps: advects the drifters of the last
  * step of members that ran all of them, then makes buffer set 0 the current
  * state again (swaps members whose block had an odd number of steps).
