@@ -224,7 +224,7 @@ struct MarchCall {
 // it since the run began): any north angle, land, dry and shallow cells,
 // one_dimensional.  Slopes of row j, flux through its south face, right-hand
 // side of row j-1 (valid from n = 4 on), and the state one row further.
-__device__ __noinline__ void march_row_general(MarchSmem& S, MarchCall& call) {
+static __device__ __noinline__ void march_row_general(MarchSmem& S, MarchCall& call) {
     const GocCdklmParams& p = S.m.p;
     const StepConst& k = S.m.k;
     const MarchOps o{S.m.c};
@@ -408,7 +408,8 @@ __device__ __forceinline__ float march_friction(const GocCdklmParams& p, float d
     return dt * p.r * sqrtf(u * u + v * v) / hs;
 }
 
-// Output rows [row0, row1) of the strip's columns: one RK2 step of length dt.
+// Output rows [row0, row1) of the strip's columns (row0 = 2 or at least 4):
+// one RK2 step of length dt.
 // p, k, c: the scalar parameters, in the kernel's parameter space or equal to
 // S.m; pm: the member's own (textures).  Called by the two warps of a strip
 // together, with S.grid and S.m set and a barrier since.
@@ -602,7 +603,7 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
 
         // ---- balanced x slope of row L and its depth check ----
         float2 wE, xE;
-        {
+        if (n >= 4) {
             const float2 vs = mul2(s.vL, su), f = at(FC, oL), fv = mul2(vs, f);
             const float2 eM = shfl_prev_y(s.eL), eP = shfl_next_x(s.eL);
             const float2 fM = shfl_prev_y(fv), fP = shfl_next_x(fv);
@@ -627,7 +628,7 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
                 bad_x = bad_x || dry(0, Kx.x, dxf.x, s.vL.x, s.eL.x, HW.x, HE.x) ||
                         dry(1, Kx.y, dxf.y, s.vL.y, s.eL.y, HW.y, HE.y);
             }
-            bad = bad || (bad_x && n >= 4);
+            bad = bad || bad_x;
         }
         bool slow = any_lane(bad);
         if (!second) {
@@ -682,27 +683,29 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
                 s.g0 = g0; s.g1 = g1; s.g2 = g2;
                 s.fuL = s.fuC; s.fuC = fuU;
                 // ---- x slopes and fluxes, right-hand side of row L ----
-                const float2 u = s.uL, v = s.vL;
-                const float2 uM = shfl_prev_y(u), uP = shfl_next_x(u);
-                const float2 vM = shfl_prev_y(v), vP = shfl_next_x(v);
-                const float2 xu = o.minmod(mul2(o.sub(u, uM), c.theta), mul2(o.sub(uP, uM), c.half), mul2(o.sub(uP, u), c.theta));
-                const float2 xv = o.minmod(mul2(o.sub(v, vM), c.theta), mul2(o.sub(vP, vM), c.half), mul2(o.sub(vP, v), c.theta));
-                const float2 HW = at(HW_, oL), HE = shfl_next_x(HW);
-                const float2 pU = shfl_next_x(fma2(xu, c.nhalf, u)), pV = shfl_next_x(fma2(xv, c.nhalf, v));
-                const float2 pE = shfl_next_x(wE);
-                float2 F0, F1, F2;
-                o.flux(xE, fma2(xu, c.half, u), fma2(xv, c.half, v), o.add(xE, HE), pE, pU, pV, o.add(pE, HE), F0, F1, F2);
-                R.fd0 = o.add(mul2(o.sub(F0, shfl_prev_y(F0)), c.inv_dx), R.fd0);
-                const float2 fd1 = o.add(mul2(o.sub(F1, shfl_prev_y(F1)), c.inv_dx), fy1);
-                const float2 fd2 = o.add(mul2(o.sub(F2, shfl_prev_y(F2)), c.inv_dx), fy2);
-                const float2 hsum = plain_add(s.eL, R.Hm), f = at(FC, oL);
-                R.e = s.eL;
-                R.hu = mul2(u, hsum);
-                R.hv = mul2(v, hsum);
-                const float2 eX = mul2(c.half, o.add(wE, xE));
-                const float2 bathx = mul2(mul2(mul2(c.g, o.add(eX, R.Hm)), o.sub(HE, HW)), c.inv_dx);
-                R.r1 = o.sub(o.add(o.add(pr(wind_X), mul2(f, R.hv)), bathx), fd1);
-                R.r2 = o.sub(o.add(o.sub(pr(wind_Y), mul2(f, R.hu)), bathy), fd2);
+                if (n >= 4) {
+                    const float2 u = s.uL, v = s.vL;
+                    const float2 uM = shfl_prev_y(u), uP = shfl_next_x(u);
+                    const float2 vM = shfl_prev_y(v), vP = shfl_next_x(v);
+                    const float2 xu = o.minmod(mul2(o.sub(u, uM), c.theta), mul2(o.sub(uP, uM), c.half), mul2(o.sub(uP, u), c.theta));
+                    const float2 xv = o.minmod(mul2(o.sub(v, vM), c.theta), mul2(o.sub(vP, vM), c.half), mul2(o.sub(vP, v), c.theta));
+                    const float2 HW = at(HW_, oL), HE = shfl_next_x(HW);
+                    const float2 pU = shfl_next_x(fma2(xu, c.nhalf, u)), pV = shfl_next_x(fma2(xv, c.nhalf, v));
+                    const float2 pE = shfl_next_x(wE);
+                    float2 F0, F1, F2;
+                    o.flux(xE, fma2(xu, c.half, u), fma2(xv, c.half, v), o.add(xE, HE), pE, pU, pV, o.add(pE, HE), F0, F1, F2);
+                    R.fd0 = o.add(mul2(o.sub(F0, shfl_prev_y(F0)), c.inv_dx), R.fd0);
+                    const float2 fd1 = o.add(mul2(o.sub(F1, shfl_prev_y(F1)), c.inv_dx), fy1);
+                    const float2 fd2 = o.add(mul2(o.sub(F2, shfl_prev_y(F2)), c.inv_dx), fy2);
+                    const float2 hsum = plain_add(s.eL, R.Hm), f = at(FC, oL);
+                    R.e = s.eL;
+                    R.hu = mul2(u, hsum);
+                    R.hv = mul2(v, hsum);
+                    const float2 eX = mul2(c.half, o.add(wE, xE));
+                    const float2 bathx = mul2(mul2(mul2(c.g, o.add(eX, R.Hm)), o.sub(HE, HW)), c.inv_dx);
+                    R.r1 = o.sub(o.add(o.add(pr(wind_X), mul2(f, R.hv)), bathx), fd1);
+                    R.r2 = o.sub(o.add(o.sub(pr(wind_Y), mul2(f, R.hu)), bathy), fd2);
+                }
                 s.eL = s.eC; s.uL = s.uC; s.vL = s.vC;
                 s.eC = eU; s.uC = uU; s.vC = vU;
             }
