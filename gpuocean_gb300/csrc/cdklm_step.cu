@@ -63,33 +63,53 @@ static int launch_members(const GocCdklmParams* p, const StepConst& k, float dt,
     return check_launch("cdklm_members_kernel");
 }
 
-template <int NSTAGE, bool CF, bool SF, bool ANGLE = false>
+// TX, TY, NT: output tile and threads per CTA.
+template <int NSTAGE, bool CF, bool SF, bool ANGLE = false, int TX = kTX, int TY = kTY, int NT = kNT>
 static int launch_tile(const GocCdklmParams* p, const StepConst& k, float dt, int rk_step,
                        const float* e0, const float* hu0, const float* hv0, float* e1, float* hu1, float* hv1,
                        float* ea, float* hua, float* hva, int pitch_f, const float* Hi, int hi_pitch_f,
                        const float* Hm, int hm_pitch_f, cudaStream_t st) {
     constexpr int HALO = 2 * NSTAGE;
-    constexpr int W = kTX + 2 * HALO, H = kTY + 2 * HALO;
+    constexpr int W = TX + 2 * HALO, H = TY + 2 * HALO;
     constexpr size_t smem = ANGLE ? sizeof(TileSmemAngle<W, H>) : sizeof(TileSmem<W, H>);
-    auto kern = cdklm_tile_kernel<kTX, kTY, NSTAGE, kNT, CF, SF, ANGLE>;
+    auto kern = cdklm_tile_kernel<TX, TY, NSTAGE, NT, CF, SF, ANGLE>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return set_error(GOC_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
         configured = true;
     }
-    dim3 grid((p->nx + kTX - 1) / kTX, (p->ny + kTY - 1) / kTY);
-    kern<<<grid, kNT, smem, st>>>(*p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi,
+    dim3 grid((p->nx + TX - 1) / TX, (p->ny + TY - 1) / TY);
+    kern<<<grid, NT, smem, st>>>(*p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi,
                                   hi_pitch_f, Hm, hm_pitch_f);
     count_launch();
     return check_launch("cdklm_tile_kernel");
 }
+
+constexpr int kSMs = 152;   // of a GB300
 
 template <int NSTAGE>
 static int dispatch(const GocCdklmParams* p, const StepConst& k, bool cf, bool sf, float dt, int rk_step,
                     const float* e0, const float* hu0, const float* hv0, float* e1, float* hu1, float* hv1,
                     float* ea, float* hua, float* hva, int pitch_f, const float* Hi, int hi_pitch_f,
                     const float* Hm, int hm_pitch_f, cudaStream_t st) {
+    if constexpr (NSTAGE == 2) {
+        // A step of a grid that leaves SMs idle, or one CTA on each, lasts as
+        // long as one CTA does: with 256 threads 14.5 us from 64 x 64 to 256 x
+        // 256.  Such grids take more threads per tile, the smallest (whose 16 x
+        // 8 tiles still find an SM each) smaller tiles as well, staged by one
+        // pass of 384 threads: 64 x 64 8.3 us, 200 x 180 and 256 x 256 10.4 us.
+        // Three simulators at once: 5.6 -> 4.0, 6.2 -> 4.6 and 6.6 -> 6.0 us a
+        // step.  With two CTAs on an SM (512 x 300) the larger CTAs gain 2 us
+        // alone and lose 1 of 10 us with others, so those keep 256 threads.
+        const long long tiles = (long long)((p->nx + kTX - 1) / kTX) * ((p->ny + kTY - 1) / kTY);
+        if (sf && tiles <= kSMs / 4)
+            return cf ? launch_tile<2, true, true, false, 16, 8, 384>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st)
+                      : launch_tile<2, false, true, false, 16, 8, 384>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st);
+        if (sf && tiles <= kSMs)
+            return cf ? launch_tile<2, true, true, false, kTX, kTY, 1024>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st)
+                      : launch_tile<2, false, true, false, kTX, kTY, 1024>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st);
+    }
     if (cf && sf)
         return launch_tile<NSTAGE, true, true>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st);
     if (cf)
