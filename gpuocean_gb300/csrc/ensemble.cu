@@ -8,6 +8,8 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <functional>
+#include <queue>
 
 #include "ensemble.cuh"
 
@@ -289,40 +291,100 @@ static bool host_tile_on_border(const GocCdklmParams& p, int tx, int ty, int i, 
     return x0 < 2 || y0 < 2 || x0 + tx + 8 > p.nx + 2 || y0 + ty + 8 > p.ny + 2;
 }
 
-// Units of kMarchShape's rows per run of the marching kernel: a run costs its
-// rows plus about four (the rows below and above it that it computes again),
-// so runs are as long as leaves about four per resident warp to even out the
-// end of the launch.
-static int build_march(Ensemble* e) {
-    cudaFree(e->d_march);
-    e->d_march = nullptr;
-    e->n_march = 0;
-    int grid = 0;
-    const int rc = ensemble_march_configure(e, &grid);
-    if (rc) return rc;
+// Runs of the marching kernel.  A run lasts its rows and about nine more (the
+// pipeline of the two stages), a row some 0.79 + 0.16 c us with c strips on
+// an SM (measured with 4, 5 and 8: 1.43, 1.55, 2.07 us).  Every CTA takes the
+// next run from the queue, longest first, so the launch ends with the run
+// that ends last: with runs of one length and hardly more runs than CTAs it
+// takes twice the time of one run.  The plan tries run lengths and, for each,
+// shorter runs for the strips at the end of the queue, plays the queue
+// through and keeps the shortest.
+struct MarchPlan {
+    int rows_most = 1;      // units per run
+    int tail_most = 1;      // ... of the strips in the tail
+    long long tail = 0;     // strips (last in member order) in the tail
+};
+
+static std::vector<int4> march_runs(const Ensemble* e, const MarchPlan& plan, long long n_strips) {
     const TileShape sh = kEnsembleShapes[kMarchShape];
-    long long units = 0;
-    for (const GocMemberDesc& d : e->host)
-        units += (long long)((d.p.nx + sh.tx - 1) / sh.tx) * ((d.p.ny + sh.ty - 1) / sh.ty);
-    const int most = (int)std::min(16LL, std::max(1LL, units / (4LL * grid)));
     std::vector<int4> runs;
+    long long s = 0;
     for (int m = 0; m < e->n_members; ++m) {
         const GocCdklmParams& p = e->host[m].p;
         const int strips = (p.nx + sh.tx - 1) / sh.tx, len = (p.ny + sh.ty - 1) / sh.ty;
-        const int n = (len + most - 1) / most;
-        for (int i = 0; i < strips; ++i)
+        for (int i = 0; i < strips; ++i, ++s) {
+            const int most = s >= n_strips - plan.tail ? plan.tail_most : plan.rows_most;
+            const int n = (len + most - 1) / most;
             for (int r = 0, j = 0; r < n; ++r) {
                 const int w = len / n + (r < len % n ? 1 : 0);
                 runs.push_back(make_int4(m, i, j, w));
                 j += w;
             }
+        }
     }
     std::stable_sort(runs.begin(), runs.end(), [](const int4& a, const int4& b) { return a.w > b.w; });
-    cudaError_t err = cudaMalloc(&e->d_march, sizeof(int4) * runs.size());
+    return runs;
+}
+
+// Time (us) of the queue on `ctas` CTAs, `per_sm` of them on an SM at most.
+static double march_makespan(const std::vector<int4>& runs, int ctas, int per_sm) {
+    const int rows = kEnsembleShapes[kMarchShape].ty;
+    const double c = std::min<double>(per_sm, (double)runs.size() * per_sm / ctas);
+    std::priority_queue<int, std::vector<int>, std::greater<int>> ends;
+    int last = 0;
+    for (const int4& r : runs) {
+        int t = r.w * rows + 9;
+        if ((int)ends.size() == ctas) {
+            t += ends.top();
+            ends.pop();
+        }
+        ends.push(t);
+        last = std::max(last, t);
+    }
+    return last * (0.79 + 0.16 * c);
+}
+
+static int build_march(Ensemble* e) {
+    cudaFree(e->d_march);
+    e->d_march = nullptr;
+    e->n_march = 0;
+    int grid = 0, dev = 0, sms = 1;
+    const int rc = ensemble_march_configure(e, &grid);
+    if (rc) return rc;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const TileShape sh = kEnsembleShapes[kMarchShape];
+    long long units = 0, strips = 0;
+    for (const GocMemberDesc& d : e->host) {
+        const long long n = (d.p.nx + sh.tx - 1) / sh.tx;
+        strips += n;
+        units += n * ((d.p.ny + sh.ty - 1) / sh.ty);
+    }
+    std::vector<int4> best;
+    double best_t = 0.0;
+    const int lengths[] = {16, 12, 8, 6, 5, 4, 3, 2, 1};
+    for (int most : lengths) {
+        // shorter runs than leave some 16 for every CTA only cost rows
+        if (most < 16 && units / most > 16LL * grid) break;
+        for (int tail = 0; tail < 3; ++tail) {
+            // the tail: about half a run or a run of every CTA
+            const double per_strip = (double)units / strips;
+            const MarchPlan plan{most, std::max(1, most / 3),
+                                 std::min(strips, (long long)(tail * 0.5 * grid * most / per_strip))};
+            if (tail && (most == 1 || plan.tail == 0)) continue;
+            std::vector<int4> runs = march_runs(e, plan, strips);
+            const double t = march_makespan(runs, grid, std::max(1, grid / sms));
+            if (best.empty() || t < best_t) {
+                best.swap(runs);
+                best_t = t;
+            }
+        }
+    }
+    cudaError_t err = cudaMalloc(&e->d_march, sizeof(int4) * best.size());
     if (err == cudaSuccess)
-        err = cudaMemcpy(e->d_march, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice);
+        err = cudaMemcpy(e->d_march, best.data(), sizeof(int4) * best.size(), cudaMemcpyHostToDevice);
     if (err != cudaSuccess) return set_error(GOC_ERR_CUDA, "ensemble march queue: %s", cudaGetErrorString(err));
-    e->n_march = (int)runs.size();
+    e->n_march = (int)best.size();
     return GOC_OK;
 }
 

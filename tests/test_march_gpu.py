@@ -99,3 +99,24 @@ def test_march_of_unlike_members(gpu_ctx):
     for a, b in zip(*out):
         for x, y in zip(a, b):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("counts", [(1, 0), (40, 3), (150, 20)])
+def test_march_queue(gpu_ctx, counts):
+    """The queue's plan from few runs (fewer than the CTAs) to many (with
+    shorter runs at its end): every cell of every member is stepped once."""
+    from gpuocean_gb300.ensembles.BatchedEnsemble import BatchedEnsemble
+    grids = [(64, 203)] * counts[0] + [(200, 88)] * counts[1]
+    out = []
+    for march in (False, True):
+        sims = [_sim(gpu_ctx, nx, ny, CHANNEL, i % 5, beta=2e-11) for i, (nx, ny) in enumerate(grids)]
+        ens = BatchedEnsemble(sims, autotune=False)
+        if march:
+            _march(ens)
+        ens.step(1.3)
+        ens.synchronize()
+        out.append(_states(sims, False))
+        ens.release()
+    for a, b in zip(*out):
+        for x, y in zip(a, b):
+            assert np.array_equal(x, y)
