@@ -422,7 +422,7 @@ struct NoiseBatch {
     int4* d_pert_items = nullptr;
     int4* d_rng_chunks = nullptr;
     curandStateXORWOW_t* d_states = nullptr;
-    int n_soar = 0, n_pert = 0, n_rng = 0, n_states = 0;
+    int n_soar = 0, n_pert = 0, n_rows = 0, n_rng = 0, n_states = 0;
 };
 
 extern "C" int goc_noise_batch_create(void* ensemble, const GocNoiseDesc* noise, void** out) {
@@ -432,7 +432,7 @@ extern "C" int goc_noise_batch_create(void* ensemble, const GocNoiseDesc* noise,
     const GocMemberDesc* members = ensemble_host_members(ensemble, &n_members);
     NoiseBatch* b = new NoiseBatch();
     b->n = n_members;
-    std::vector<int4> soar, pert, rng;
+    std::vector<int4> soar, pert, rows, rng;
     int states = 0;
     for (int m = 0; m < n_members; ++m) {
         int rc = check_noise(&noise[m], "goc_noise_batch_create");
@@ -446,8 +446,10 @@ extern "C" int goc_noise_batch_create(void* ensemble, const GocNoiseDesc* noise,
         }
         for (int j = 0; j < (noise[m].coarse_ny + 4 + kNB - 1) / kNB; ++j)
             for (int i = 0; i < (noise[m].coarse_nx + 4 + kNB - 1) / kNB; ++i) soar.push_back(make_int4(m, i, j, 0));
-        for (int j = 0; j < (md.p.ny + kPY - 1) / kPY; ++j)
-            for (int i = 0; i < (md.p.nx + kPX - 1) / kPX; ++i) pert.push_back(make_int4(m, i, j, 0));
+        const bool by_rows = perturb_by_rows(noise[m], md.p.dx, md.p.dy, md.p.ny, md.pitch, md.Hi_pitch);
+        const int tx = by_rows ? kRX : kPX, ty = by_rows ? kRY : kPY;
+        for (int j = 0; j < (md.p.ny + ty - 1) / ty; ++j)
+            for (int i = 0; i < (md.p.nx + tx - 1) / tx; ++i) (by_rows ? rows : pert).push_back(make_int4(m, i, j, 0));
         const int rnx = noise[m].periodic_ew ? noise[m].coarse_nx : noise[m].coarse_nx + 8;
         const int rny = noise[m].periodic_ns ? noise[m].coarse_ny : noise[m].coarse_ny + 8;
         for (int f = 0; f < rnx * rny; f += 256) {
@@ -458,6 +460,8 @@ extern "C" int goc_noise_batch_create(void* ensemble, const GocNoiseDesc* noise,
     }
     b->n_soar = (int)soar.size();
     b->n_pert = (int)pert.size();
+    b->n_rows = (int)rows.size();
+    pert.insert(pert.end(), rows.begin(), rows.end());
     b->n_rng = (int)rng.size();
     b->n_states = states;
     cudaError_t e = cudaMalloc(&b->d_noise, sizeof(GocNoiseDesc) * n_members);
@@ -546,7 +550,7 @@ extern "C" int goc_noise_batch_perturb(void* batch, void* ensemble, float pertur
     count_launch();
     int rc = check_launch("soar_batched_active_kernel");
     if (rc) return rc;
-    return launch_perturb_batched(b->d_noise, ensemble_device_members(ensemble), b->d_pert_items, b->n_pert, nsub,
+    return launch_perturb_batched(b->d_noise, ensemble_device_members(ensemble), b->d_pert_items, b->n_pert, b->n_rows, nsub,
                                   substep, st);
 }
 

@@ -30,21 +30,26 @@ __device__ __forceinline__ OceanRef ocean_of(const GocMemberDesc& m, int images)
                     m.p.land_value, images && m.p.bc_north == 2, images && m.p.bc_east == 2};
 }
 
-// Write a perturbed interior cell and, for periodic boundaries, its ghost
-// images (the boundary fill the reference runs after perturbState,
+// Write a perturbed interior cell's ghost images for periodic boundaries
+// (the boundary fill the reference runs after perturbState,
 // S/CDKLM16.py:571-572).
+__device__ __forceinline__ void store_images(const OceanRef& o, int ti, int tj, float e, float u, float v) {
+    const int x = !o.images_ew ? -1 : ti < 4 ? ti + o.nx : ti >= o.nx ? ti - o.nx : -1;
+    const int y = !o.images_ns ? -1 : tj < 4 ? tj + o.ny : tj >= o.ny ? tj - o.ny : -1;
+    auto store = [&](int yy, int xx) {
+        const size_t k = (size_t)yy * o.pitch + xx;
+        o.eta[k] = e; o.hu[k] = u; o.hv[k] = v;
+    };
+    if (x >= 0) store(tj, x);
+    if (y >= 0) store(y, ti);
+    if (x >= 0 && y >= 0) store(y, x);
+}
+
+// ... and the cell itself.
 __device__ __forceinline__ void store_cell(const OceanRef& o, int ti, int tj, float e, float u, float v) {
-    int xs[2] = {ti, -1}, ys[2] = {tj, -1};
-    if (o.images_ew) xs[1] = (ti < 4) ? ti + o.nx : (ti >= o.nx ? ti - o.nx : -1);
-    if (o.images_ns) ys[1] = (tj < 4) ? tj + o.ny : (tj >= o.ny ? tj - o.ny : -1);
-    for (int a = 0; a < 2; ++a) {
-        if (ys[a] < 0) continue;
-        for (int b = 0; b < 2; ++b) {
-            if (xs[b] < 0) continue;
-            const size_t k = (size_t)ys[a] * o.pitch + xs[b];
-            o.eta[k] = e; o.hu[k] = u; o.hv[k] = v;
-        }
-    }
+    const size_t k = (size_t)tj * o.pitch + ti;
+    o.eta[k] = e; o.hu[k] = u; o.hv[k] = v;
+    store_images(o, ti, tj, e, u, v);
 }
 
 // Coriolis parameter of cell (ti, tj) as the noise kernels see it: f plus the
@@ -91,12 +96,13 @@ __device__ __forceinline__ int bicubic_cj(const GocNoiseDesc& d, float dy, int t
     return cj;
 }
 
-__device__ __forceinline__ void bicubic_coeffs(const GocNoiseDesc& d, int ci, int cj, float* A /* [16], row-major */) {
+// Column q of the 4x4 coefficients A = B F B^T of coarse cell (ci, cj).
+__device__ __forceinline__ float4 bicubic_column(const GocNoiseDesc& d, int ci, int cj, int q) {
     float c[4][4];  // c[row][col] = coarse[cj-1+row][ci-1+col]
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) c[r][q] = coarse_at(d, cj - 1 + r, ci - 1 + q);
+        for (int k = 0; k < 4; ++k) c[r][k] = coarse_at(d, cj - 1 + r, ci - 1 + k);
     // values, x/y derivatives and cross derivatives at the 4 corners
     float F[4][4];
     F[0][0] = c[1][1]; F[0][1] = c[2][1]; F[1][0] = c[1][2]; F[1][1] = c[2][2];
@@ -109,17 +115,23 @@ __device__ __forceinline__ void bicubic_coeffs(const GocNoiseDesc& d, int ci, in
     F[2][2] = (F[1][2] - fy_10) / 2.0f; F[2][3] = (F[1][3] - fy_11) / 2.0f;
     F[3][2] = (fy20 - F[0][2]) / 2.0f; F[3][3] = (fy21 - F[0][3]) / 2.0f;
     const float B[4][4] = {{1, 0, 0, 0}, {0, 0, 1, 0}, {-3, 3, -2, -1}, {2, -2, 1, 1}};
-    float FB[4][4];   // FB = F B^T, A = B FB
+    const float b[4] = {q == 0 ? 1.0f : q == 2 ? -3.0f : q == 3 ? 2.0f : 0.0f,      // B[q]
+                        q == 2 ? 3.0f : q == 3 ? -2.0f : 0.0f,
+                        q == 0 ? 0.0f : q == 2 ? -2.0f : 1.0f, q == 2 ? -1.0f : q == 3 ? 1.0f : 0.0f};
+    float FB[4], A[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < 4; ++r) FB[r] = F[r][0] * b[0] + F[r][1] * b[1] + F[r][2] * b[2] + F[r][3] * b[3];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            FB[r][q] = F[r][0] * B[q][0] + F[r][1] * B[q][1] + F[r][2] * B[q][2] + F[r][3] * B[q][3];
+    for (int r = 0; r < 4; ++r) A[r] = B[r][0] * FB[0] + B[r][1] * FB[1] + B[r][2] * FB[2] + B[r][3] * FB[3];
+    return make_float4(A[0], A[1], A[2], A[3]);
+}
+
+__device__ __forceinline__ void bicubic_coeffs(const GocNoiseDesc& d, int ci, int cj, float* A /* [16], row-major */) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            A[4 * r + q] = B[r][0] * FB[0][q] + B[r][1] * FB[1][q] + B[r][2] * FB[2][q] + B[r][3] * FB[3][q];
+    for (int q = 0; q < 4; ++q) {
+        const float4 a = bicubic_column(d, ci, cj, q);
+        A[q] = a.x; A[4 + q] = a.y; A[8 + q] = a.z; A[12 + q] = a.w;
+    }
 }
 
 __device__ __forceinline__ float bicubic_eval(const float* A, float rx, float ry) {
@@ -198,21 +210,20 @@ __device__ __forceinline__ void perturbed_state(const GocNoiseDesc& d, int nx, i
     const float H_mid = 0.25f * (hc[0] + hc[1] + hc[2] + hc[3]);
     const float cor = noise_coriolis(d, nx, ny, dx, dy, ti, tj);
     const float dc = de(tj, ti);
-    const float ex = (de(tj, ti + 1) - de(tj, ti - 1)) / (2.0f * dx);
-    const float ey = (de(tj + 1, ti) - de(tj - 1, ti)) / (2.0f * dy);
+    // reciprocals of the steps: at most 1.5 ulp a quotient, the division's 2
+    const float ex = (de(tj, ti + 1) - de(tj, ti - 1)) * (1.0f / (2.0f * dx));
+    const float ey = (de(tj + 1, ti) - de(tj - 1, ti)) * (1.0f / (2.0f * dy));
+    const float gc = __fdividef(d.g, cor);
     if (factor1) {
-        const float h_mid = dc + H_mid + e;
-        const float dhu = -(d.g / cor) * h_mid * ey;
-        const float dhv = (d.g / cor) * h_mid * ex;
+        const float gH = gc * (dc + H_mid + e);
         if (dry) {
             e = 0.0f; u = 0.0f; v = 0.0f;
         } else {
-            e += dc; u += dhu; v += dhv;
+            e += dc; u -= gH * ey; v += gH * ex;
         }
     } else if (!dry) {
-        e += dc;
-        u += -(d.g / cor) * (H_mid + dc) * ey;
-        v += (d.g / cor) * (H_mid + dc) * ex;
+        const float gH = gc * (H_mid + dc);
+        e += dc; u -= gH * ey; v += gH * ex;
     }
 }
 
@@ -230,14 +241,30 @@ inline int make_ocean(int nx, int ny, float dx, float dy, float* eta, float* hu,
 }
 
 // Tiles of the stand-alone transfer kernels (noise_transfer.cu): kPX x kPY
-// interior cells, kPT thread rows of kPX threads.
+// interior cells, kPT thread rows of kPX threads; or kRX x kRY interior cells
+// for the members that perturb_by_rows picks.
 constexpr int kPX = 32, kPY = 32, kPT = 8;
+constexpr int kRX = 60, kRY = 32;
+constexpr int kRowsCoarseX = 16, kRowsCoarseY = 10;     // coarse cells that a kRX x kRY tile and its ring may cross
+
+// Whether a member's transfer takes the kernel whose warps march: bicubic
+// up-sampling, no Coriolis texture (its look-ups would stay in the registers
+// of every row: 12.3 us against the tile kernel's 8.2, 512 x 300), a coarse
+// grid of factor 5 or coarser (at factor 3 the tables take longer than they
+// save: 8.2 us against 7.2, 512 x 300; the interpolation factor promises the
+// coarse grid but does not force it), and arrays that 32-bit indices reach.
+inline bool perturb_by_rows(const GocNoiseDesc& d, float dx, float dy, int ny, int pitch, int Hi_pitch) {
+    return d.interpolation_factor > 1 && !(d.f == 0.0f && d.coriolis_f) &&
+           (kRX + 1) * dx <= (kRowsCoarseX - 3) * d.coarse_dx && (kRY + 1) * dy <= (kRowsCoarseY - 3) * d.coarse_dy &&
+           (ny + 5LL) * (pitch > Hi_pitch ? pitch : Hi_pitch) / 4 < (1LL << 31);
+}
 
 // Stand-alone transfer of every member's coarse field after RK2 step
 // `substep` of a block (substep < 0: between blocks), one tile per item
-// (member, tile column, tile row, -) (noise_transfer.cu).
+// (member, tile column, tile row, -): n_items tiles of kPX x kPY, then n_rows
+// tiles of kRX x kRY (noise_transfer.cu).
 int launch_perturb_batched(const GocNoiseDesc* noise, const GocMemberDesc* members, const int4* items, int n_items,
-                           const int* nsub, int substep, cudaStream_t stream);
+                           int n_rows, const int* nsub, int substep, cudaStream_t stream);
 
 // substep < 0: between blocks, the state of member m is buffer set 0 of the
 // ensemble's device member table (-1: every member; -2: the members that
