@@ -14,7 +14,9 @@ different numbers of steps; a member whose block is done idles.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
+import operator
 
 import numpy as np
 
@@ -24,6 +26,8 @@ from ..utils import Common
 
 # member grid signature -> index of the fastest tile shape (per process)
 _AUTOTUNE_CACHE = {}
+# a simulator's current state buffer, by which the engine sees that members were swapped or replaced
+_state_address = operator.attrgetter("gpu_data.h0.data.ptr")
 
 
 class GocMemberDesc(ctypes.Structure):
@@ -107,6 +111,7 @@ class BatchedEnsemble:
         self._handle = None
         self._noise = None
         self._noise_kind = None
+        self._moment_bufs = collections.deque()     # device buffers of moments() between calls, two at most
         self._noises = None
         self._noise_sources = None
         self._rng_seed = None
@@ -169,7 +174,7 @@ class BatchedEnsemble:
         return descs
 
     def _current_ptrs(self):
-        return tuple(s.gpu_data.h0.ptr for s in self.sims)
+        return tuple(map(_state_address, self.sims))
 
     def _build(self, max_substeps=8):
         self._release_handles()
@@ -318,6 +323,8 @@ class BatchedEnsemble:
 
     def _release_handles(self):
         self.release_noise()
+        while getattr(self, "_moment_bufs", None):
+            self._moment_bufs.popleft().free()
         for name in ("_obs_pos", "_obs_out", "_drift_gather", "_obs_scatter"):
             buf = getattr(self, name, None)
             if buf is not None:
@@ -840,8 +847,11 @@ class BatchedEnsemble:
         s0 = self.sims[first]
         planes = 3 if quantity == "state" else 2
         nbytes = 4 * planes * int(s0.nx) * int(s0.ny)
-        bm = Common.DevicePtr(nbytes) if mean else None
-        bv = Common.DevicePtr(nbytes) if var else None
+        # allocating and freeing the two buffers took 170 of 390 us (96 members
+        # of 512 x 300): those that are not handed out are kept for later calls
+        new = self._take_moment_buffer if download else Common.DevicePtr
+        bm = new(nbytes) if mean else None
+        bv = new(nbytes) if var else None
         eps = 0.0 if desingularise is None else float(desingularise)
         before = _lib.load().goc_kernel_launch_count()
         _lib.call("goc_ensemble_moments", self._handle, int(first), count, 0 if quantity == "state" else 1,
@@ -850,14 +860,30 @@ class BatchedEnsemble:
         if not download:
             return bm, bv
         shape = (planes, int(s0.ny), int(s0.nx))
-        out = []
+        out = tuple(None if b is None else self._download(b, shape) for b in (bm, bv))
         for b in (bm, bv):
-            if b is None:
-                out.append(None)
-            else:
-                out.append(self._download(b, shape))
-                b.free()
-        return tuple(out)
+            if b is not None:
+                self._put_moment_buffer(b)
+        return out
+
+    def _take_moment_buffer(self, nbytes):
+        """A device buffer of at least nbytes: one put back by an earlier call
+        if it is large enough.  A call that runs meanwhile on another thread
+        finds it gone and takes its own."""
+        while True:
+            try:
+                buf = self._moment_bufs.popleft()
+            except IndexError:
+                return Common.DevicePtr(nbytes)
+            if buf.nbytes >= nbytes:
+                return buf
+            buf.free()
+
+    def _put_moment_buffer(self, buf):
+        if len(self._moment_bufs) < 2:
+            self._moment_bufs.append(buf)
+        else:
+            buf.free()
 
     def max_dt(self):
         """Per member the CFL limit 0.25 min(dx / |u +- c|, dy / |v +- c|)
