@@ -63,8 +63,10 @@ __global__ void observe_members_kernel(const GocMemberDesc* __restrict__ mem, in
 // ensemble moments
 // ---------------------------------------------------------------------------
 
-constexpr int kMX = 32, kMY = 8;       // cells per block
+constexpr int kMX = 32, kMY = 4;       // threads per block; each owns two neighbouring cells of a row
 constexpr int kMChunk = 128;           // member pointers staged in shared memory at a time
+constexpr int kMBlocks = 2;            // blocks per SM to have before the members are not sliced
+constexpr int kMUnroll = 8;            // members whose loads are in flight together
 
 struct MomentSrc {
     const float* a; const float* b; const float* c;  // eta, hu, hv of buffer set 0
@@ -93,28 +95,70 @@ __device__ __forceinline__ void member_values(const MomentSrc& s, int x, int y, 
     }
 }
 
-// One slice of the members: shifted sums s1 = sum(x - K), s2 = sum((x - K)^2)
-// with K the first member's value.  With one slice the moments are written
-// directly; otherwise the per-slice sums go to `part` (slice, 2P, cells).
+// The arrays of one member at cells x and x + 1 (the second may be a ghost
+// cell), as loaded; WIDE: rows start on 8-byte boundaries.
+template <int Q, bool WIDE>
+__device__ __forceinline__ void load_pair(const MomentSrc& s, int x, int y, float2* v) {
+    auto pair = [](const float* p) {
+        return WIDE ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(__ldg(p), __ldg(p + 1));
+    };
+    const size_t k = (size_t)(y + 2) * s.pitch + (x + 2);
+    v[0] = pair(s.a + k); v[1] = pair(s.b + k); v[2] = pair(s.c + k);
+    if (Q == 1) v[3] = pair(s.Hm + (size_t)(y + 2) * s.Hm_pitch + (x + 2));
+}
+
+// ... and the quantities from them.
 template <int Q>
+__device__ __forceinline__ void pair_values(const float2* v, float eps, float2* out) {
+    if (Q == 0) {
+        out[0] = v[0]; out[1] = v[1]; out[2] = v[2];
+    } else {
+        const float h0 = __fadd_rn(v[0].x, v[3].x), h1 = __fadd_rn(v[0].y, v[3].y);
+        out[0] = make_float2(desingularised_velocity(h0, v[1].x, eps), desingularised_velocity(h1, v[1].y, eps));
+        out[1] = make_float2(desingularised_velocity(h0, v[2].x, eps), desingularised_velocity(h1, v[2].y, eps));
+    }
+}
+
+// s += a with what the rounding lost kept in c (Kahan): the members' sums
+// would else run longer than those of a slice did.
+__device__ __forceinline__ void add_to(float2& s, float2& c, float2 a) {
+    const float2 y = make_float2(__fsub_rn(a.x, c.x), __fsub_rn(a.y, c.y));
+    const float2 t = make_float2(__fadd_rn(s.x, y.x), __fadd_rn(s.y, y.y));
+    c = make_float2(__fsub_rn(__fsub_rn(t.x, s.x), y.x), __fsub_rn(__fsub_rn(t.y, s.y), y.y));
+    s = t;
+}
+
+// One slice of the members: shifted sums s1 = sum(x - K), s2 = sum((x - K)^2)
+// with K the first member's value, kMUnroll members at a time as a tree.
+// With one slice the moments are written directly; otherwise the per-slice
+// sums go to `part` (slice, 2P, cells).
+//
+// What bounds it: HBM, given enough loads in flight: eight members' arrays of
+// two cells a thread.  96 members of 512 x 300, velocities: 39 us (6.0 TB/s); one cell a
+// thread, four members in flight and six slices took 92 us with their sum.
+template <int Q, bool WIDE>
 __global__ void __launch_bounds__(kMX * kMY) moments_kernel(const GocMemberDesc* __restrict__ mem, int first, int n,
                                                             int per_slice, int nx, int ny, float eps, int ddof,
                                                             float* __restrict__ mean, float* __restrict__ var,
                                                             float* __restrict__ part) {
-    constexpr int P = Q == 0 ? 3 : 2;
+    constexpr int P = Q == 0 ? 3 : 2, A = Q == 0 ? 3 : 4;
     __shared__ MomentSrc s_src[kMChunk];
-    const int x = blockIdx.x * kMX + threadIdx.x, y = blockIdx.y * kMY + threadIdx.y;
+    const int x = 2 * (blockIdx.x * kMX + threadIdx.x), y = blockIdx.y * kMY + threadIdx.y;
     const int t = threadIdx.y * kMX + threadIdx.x;
     const bool inside = x < nx && y < ny;
     const int m0 = blockIdx.z * per_slice, m1 = min(n, m0 + per_slice);
-    float K[P], s1[P], s2[P];
+    float2 K[P], s1[P], s2[P], lost1[P], lost2[P];
     {
         const GocMemberDesc& d = mem[first];
         const MomentSrc s{d.eta[0], d.hu[0], d.hv[0], d.Hm, d.pitch / 4, d.Hm_pitch / 4};
-        if (inside) member_values<Q>(s, x, y, eps, K);
+        float2 v[A];
+        if (inside) {
+            load_pair<Q, WIDE>(s, x, y, v);
+            pair_values<Q>(v, eps, K);
+        }
     }
 #pragma unroll
-    for (int q = 0; q < P; ++q) s1[q] = s2[q] = 0.0f;
+    for (int q = 0; q < P; ++q) s1[q] = s2[q] = lost1[q] = lost2[q] = make_float2(0.0f, 0.0f);
     for (int c0 = m0; c0 < m1; c0 += kMChunk) {
         const int cn = min(kMChunk, m1 - c0);
         __syncthreads();
@@ -125,45 +169,66 @@ __global__ void __launch_bounds__(kMX * kMY) moments_kernel(const GocMemberDesc*
         __syncthreads();
         if (!inside) continue;
         int i = 0;
-        for (; i + 4 <= cn; i += 4) {   // four members' loads in flight
-            float v[4][P];
+        for (; i + kMUnroll <= cn; i += kMUnroll) {
+            float2 v[kMUnroll][A];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) member_values<Q>(s_src[i + u], x, y, eps, v[u]);
+            for (int u = 0; u < kMUnroll; ++u) load_pair<Q, WIDE>(s_src[i + u], x, y, v[u]);
+            float2 e[kMUnroll][P];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < kMUnroll; ++u) {
+                pair_values<Q>(v[u], eps, e[u]);
 #pragma unroll
-                for (int q = 0; q < P; ++q) {
-                    const float e = v[u][q] - K[q];
-                    s1[q] += e;
-                    s2[q] += e * e;
-                }
-        }
-        for (; i < cn; ++i) {
-            float v[P];
-            member_values<Q>(s_src[i], x, y, eps, v);
+                for (int q = 0; q < P; ++q) e[u][q] = make_float2(e[u][q].x - K[q].x, e[u][q].y - K[q].y);
+            }
 #pragma unroll
             for (int q = 0; q < P; ++q) {
-                const float e = v[q] - K[q];
-                s1[q] += e;
-                s2[q] += e * e;
+                float2 a[kMUnroll], b[kMUnroll];
+#pragma unroll
+                for (int u = 0; u < kMUnroll; ++u) {
+                    a[u] = e[u][q];
+                    b[u] = make_float2(a[u].x * a[u].x, a[u].y * a[u].y);
+                }
+#pragma unroll
+                for (int w = kMUnroll / 2; w > 0; w /= 2)
+#pragma unroll
+                    for (int u = 0; u < w; ++u) {
+                        a[u] = make_float2(a[u].x + a[u + w].x, a[u].y + a[u + w].y);
+                        b[u] = make_float2(b[u].x + b[u + w].x, b[u].y + b[u + w].y);
+                    }
+                add_to(s1[q], lost1[q], a[0]);
+                add_to(s2[q], lost2[q], b[0]);
+            }
+        }
+        for (; i < cn; ++i) {
+            float2 v[A], w[P];
+            load_pair<Q, WIDE>(s_src[i], x, y, v);
+            pair_values<Q>(v, eps, w);
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                const float e0 = w[q].x - K[q].x, e1 = w[q].y - K[q].y;
+                add_to(s1[q], lost1[q], make_float2(e0, e1));
+                add_to(s2[q], lost2[q], make_float2(e0 * e0, e1 * e1));
             }
         }
     }
     if (!inside) return;
-    const size_t cells = (size_t)nx * ny, c = (size_t)y * nx + x;
-    if (part) {
-        float* o = part + (size_t)blockIdx.z * 2 * P * cells + c;
+    const size_t cells = (size_t)nx * ny;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (x + h >= nx) break;
+        const size_t c = (size_t)y * nx + x + h;
 #pragma unroll
         for (int q = 0; q < P; ++q) {
-            o[(2 * q) * cells] = s1[q];
-            o[(2 * q + 1) * cells] = s2[q];
+            const float a = h ? s1[q].y : s1[q].x, b = h ? s2[q].y : s2[q].x, k = h ? K[q].y : K[q].x;
+            if (part) {
+                float* o = part + (size_t)blockIdx.z * 2 * P * cells + c;
+                o[(2 * q) * cells] = a;
+                o[(2 * q + 1) * cells] = b;
+                continue;
+            }
+            if (mean) mean[q * cells + c] = k + __fdiv_rn(a, (float)n);
+            if (var) var[q * cells + c] = __fdiv_rn(b - __fdiv_rn(a * a, (float)n), (float)(n - ddof));
         }
-        return;
-    }
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-        if (mean) mean[q * cells + c] = K[q] + __fdiv_rn(s1[q], (float)n);
-        if (var) var[q * cells + c] = __fdiv_rn(s2[q] - __fdiv_rn(s1[q] * s1[q], (float)n), (float)(n - ddof));
     }
 }
 
@@ -292,15 +357,23 @@ extern "C" int goc_ensemble_moments(void* ensemble, int first_member, int n_memb
     if (!mean && !var) return set_error(GOC_ERR_ARG, "goc_ensemble_moments: no output");
     if (ddof < 0) return set_error(GOC_ERR_ARG, "goc_ensemble_moments: negative ddof");
     const int nx = host[first_member].p.nx, ny = host[first_member].p.ny;
-    for (int m = first_member; m < first_member + n_members; ++m)
-        if (host[m].p.nx != nx || host[m].p.ny != ny)
+    bool wide = true;       // every member's rows on 8-byte boundaries
+    for (int m = first_member; m < first_member + n_members; ++m) {
+        const GocMemberDesc& d = host[m];
+        if (d.p.nx != nx || d.p.ny != ny)
             return set_error(GOC_ERR_ARG, "goc_ensemble_moments: members %d and %d differ in grid size", first_member, m);
+        uintptr_t bits = (uintptr_t)d.Hm | (uintptr_t)d.pitch | (uintptr_t)d.Hm_pitch;
+        for (int set = 0; set < 2; ++set) bits |= (uintptr_t)d.eta[set] | (uintptr_t)d.hu[set] | (uintptr_t)d.hv[set];
+        wide = wide && (bits & 7u) == 0;
+    }
     const int P = quantity == 0 ? 3 : 2;
     const size_t cells = (size_t)nx * ny;
-    dim3 blk(kMX, kMY), grd((nx + kMX - 1) / kMX, (ny + kMY - 1) / kMY);
-    // split the members over slices until about four waves of blocks cover the device
+    dim3 blk(kMX, kMY), grd((nx + 2 * kMX - 1) / (2 * kMX), (ny + kMY - 1) / kMY);
+    // slices of the members until each SM has two blocks: fewer leave too few
+    // loads in flight, more only add sums to write and read (96 members of
+    // 512 x 300, velocities: 39 us in one slice, 46 in two, 49 in three)
     const long long blocks = (long long)grd.x * grd.y;
-    int slices = (int)std::min<long long>(std::max<long long>(1, (152LL * 8 * 4 + blocks - 1) / blocks),
+    int slices = (int)std::min<long long>(std::max<long long>(1, (152LL * kMBlocks + blocks - 1) / blocks),
                                           std::max(1, n_members / 16));
     slices = std::min(slices, 65535);
     const int per_slice = (n_members + slices - 1) / slices;
@@ -323,16 +396,13 @@ extern "C" int goc_ensemble_moments(void* ensemble, int first_member, int n_memb
     }
     grd.z = slices;
     const GocMemberDesc* dm = ensemble_device_members(ensemble);
-    if (quantity == 0)
-        moments_kernel<0><<<grd, blk, 0, st>>>(dm, first_member, n_members, per_slice, nx, ny, desing_eps, ddof,
-                                               mean, var, part);
-    else
-        moments_kernel<1><<<grd, blk, 0, st>>>(dm, first_member, n_members, per_slice, nx, ny, desing_eps, ddof,
-                                               mean, var, part);
+    const auto kernel = quantity == 0 ? (wide ? moments_kernel<0, true> : moments_kernel<0, false>)
+                                      : (wide ? moments_kernel<1, true> : moments_kernel<1, false>);
+    kernel<<<grd, blk, 0, st>>>(dm, first_member, n_members, per_slice, nx, ny, desing_eps, ddof, mean, var, part);
     count_launch();
     int rc = check_launch("moments_kernel");
     if (rc || slices == 1) return rc;
-    grd.z = 1;
+    grd = dim3((nx + kMX - 1) / kMX, (ny + kMY - 1) / kMY);
     if (quantity == 0)
         moments_finish_kernel<0><<<grd, blk, 0, st>>>(dm, first_member, n_members, slices, nx, ny, desing_eps, ddof,
                                                       part, mean, var);

@@ -116,6 +116,24 @@ def test_velocity_moments(gpu_ctx, eps):
     ens.release()
 
 
+@pytest.mark.parametrize("n,nx,ny", [(1, 21, 10), (8, 63, 12), (17, 65, 13), (33, 64, 9), (130, 31, 11)])
+def test_moments_at_the_edges(gpu_ctx, n, nx, ny):
+    """Odd and even rows (single and paired loads), one cell past a block,
+    member counts around the unrolled loop, the staged chunk and the slices,
+    against the same bars as above."""
+    ens, sims = _stepped(gpu_ctx, n, nx, ny, steps=1)
+    Hm = np.asarray(sims[0].downloadBathymetry()[1], np.float32)[2:-2, 2:-2]
+    states = _states(sims)
+    for quantity, ref in (("state", states), ("velocity", eso.velocities(states, Hm))):
+        mean, var = ens.moments(quantity=quantity)
+        ref_m, ref_v = eso.moments(ref)
+        for q in range(len(mean)):
+            assert _close(mean[q], ref_m[q], 2e-6), (quantity, q)
+            if n > 1:
+                assert _close(var[q], ref_v[q], 1e-5), (quantity, q)
+    ens.release()
+
+
 def test_multilevel_estimators(gpu_ctx):
     """Device ML estimator: with the device's own level statistics, the
     assembly equals the reference formula bit for bit; against the FP64
