@@ -268,3 +268,29 @@ def test_kl_rates_reference_per_member_vs_batched(gpu_ctx):
                       "batched_all_members_ms": 1e3 * batched, "batched_member_cells_per_s": cells / batched,
                       "speedup": n * ref_member / batched}))
     assert batched < n * ref_member
+
+
+@pytest.mark.parametrize("basis,nx,ny", [((1, 1, 1, 1), 33, 20), ((1, 64, 1, 2), 126, 30), ((3, 67, 1, 2), 127, 31),
+                                         ((1, 70, 2, 4), 255, 130), ((5, 6, 1, 40), 40, 128)])
+def test_kl_tables_against_oracle(gpu_ctx, basis, nx, ny):
+    """Table blocks: around the 64 powers that a block shares, entries around
+    the blocks of 128, single and many basis rows.  Tolerance: a phase 2 pi n x
+    carries two float32 roundings of x, 1.5e-6 n of a term of size n^-1.25;
+    some 200 such terms give 5e-6 of the field, asked for is four times that."""
+    from gpuocean_gb300.SWEsimulators.ModelErrorKL import ModelErrorKL
+    from gpuocean_gb300.utils import Common
+    rng = np.random.default_rng(nx)
+    rns = rng.standard_normal((2 * (basis[3] - basis[2] + 1), basis[1] - basis[0] + 1)).astype(np.float32)
+    rollers = tuple(float(np.float32(r)) for r in rng.uniform(size=4))
+    stream = Common.Stream()
+    me = ModelErrorKL(gpu_ctx, stream, nx, ny, 2000.0, 2500.0, Common.BoundaryConditions(), kl_decay=1.25,
+                      kl_scaling=0.025, basis_x_start=basis[0], basis_x_end=basis[1], basis_y_start=basis[2],
+                      basis_y_end=basis[3])
+    eta = Common.CUDAArray2D(stream, nx, ny, 2, 2, np.zeros((ny + 4, nx + 4), np.float32))
+    me.perturbEta(eta, random_numbers=rns, perturbation_scale=0.7, roll_x_sin=rollers[0], roll_y_sin=rollers[1],
+                  roll_x_cos=rollers[2], roll_y_cos=rollers[3])
+    got = eta.download(stream)[2:-2, 2:-2]
+    d = ko.kl_d_eta(nx, ny, rns, *basis, True, True, np.float32(1.25), np.float32(0.025), 0.7, rollers)
+    assert _rel(got, d[1:-1, 1:-1]) <= 2e-5
+    eta.release()
+    me.cleanUp()
