@@ -109,7 +109,10 @@ __device__ void stage_vjp_body(const GocCdklmParams& p, const StepConst& k, floa
             }
         }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) A.Db[c][j][i] = 0.0f;
+        for (int c = 0; c < 3; ++c) {
+            A.Db[c][j][i] = 0.0f;
+            if (HAS_Y) { S.Fx[c][j][i] = 0.0f; S.Gy[c][j][i] = 0.0f; }    // no fluxes: free for the adjoints
+        }
     }
     __syncthreads();
 
@@ -129,16 +132,16 @@ __device__ void stage_vjp_body(const GocCdklmParams& p, const StepConst& k, floa
     }
 
     // 3. cell pass: RK combination, friction and source terms in reverse.
-    //    The flux-divergence adjoints stay in registers until every cell has
-    //    read the fluxes, then replace them in the Gy planes.
+    //    The flux-divergence adjoints go to the Gy planes; without y they
+    //    wait in registers until every cell has read the fluxes there.
     float wXb = 0.0f, wYb = 0.0f;
     constexpr int NCELL = (W - 4) * (H - 4);
     constexpr int PER = (NCELL + NT - 1) / NT;
     // A rolled loop keeps one copy of the cell pass in the kernel (it is
     // sensitive to the instruction cache); fdb then lives in local memory.
-    float fdb[PER][3];
+    float fdb[HAS_Y ? 1 : PER][3];
 #pragma unroll
-    for (int r = 0; r < PER; ++r) { fdb[r][0] = 0.f; fdb[r][1] = 0.f; fdb[r][2] = 0.f; }
+    for (int r = 0; r < (HAS_Y ? 1 : PER); ++r) { fdb[r][0] = 0.f; fdb[r][1] = 0.f; fdb[r][2] = 0.f; }
 #pragma unroll 1
     for (int r = 0; r < PER; ++r) {
         const int idx = threadIdx.x + r * NT;
@@ -228,9 +231,11 @@ __device__ void stage_vjp_body(const GocCdklmParams& p, const StepConst& k, floa
         }
         float hsb = 0.0f;
         friction_vjp(p, dt, hsum, hu, hv, Cb, hsb, hub, hvb);
-        fdb[r][0] = -L1b;
-        fdb[r][1] = -L2b;
-        fdb[r][2] = -L3b;
+        if constexpr (HAS_Y) {
+            S.Gy[0][j][i] = -L1b; S.Gy[1][j][i] = -L2b; S.Gy[2][j][i] = -L3b;
+        } else {
+            fdb[r][0] = -L1b; fdb[r][1] = -L2b; fdb[r][2] = -L3b;
+        }
         const float uc = S.D[1][j][i], vc = S.D[2][j][i];
         if (hsum >= p.depth_cutoff && ec != kDryFlag) {
             const float st1b = L2b, st2b = L3b;
@@ -264,24 +269,26 @@ __device__ void stage_vjp_body(const GocCdklmParams& p, const StepConst& k, floa
         }
     }
     __syncthreads();
-    // the fluxes are dead: Gy takes the flux-divergence adjoints (zero outside
-    // the cells of the pass), Fx the slope adjoints
-    for (int idx = threadIdx.x; idx < H * W; idx += NT) {
-        const int i = idx % W, j = idx / W;
+    if constexpr (!HAS_Y) {
+        // the fluxes are dead: Gy takes the flux-divergence adjoints (zero outside
+        // the cells of the pass), Fx the slope adjoints
+        for (int idx = threadIdx.x; idx < H * W; idx += NT) {
+            const int i = idx % W, j = idx / W;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) { S.Fx[c][j][i] = 0.0f; S.Gy[c][j][i] = 0.0f; }
-    }
-    __syncthreads();
+            for (int c = 0; c < 3; ++c) { S.Fx[c][j][i] = 0.0f; S.Gy[c][j][i] = 0.0f; }
+        }
+        __syncthreads();
 #pragma unroll
-    for (int r = 0; r < PER; ++r) {
-        const int idx = threadIdx.x + r * NT;
-        if (idx >= NCELL) continue;
-        int i, j;
-        block_cell<W - 4>(idx, H - 4, i, j);
-        i += 2; j += 2;
-        S.Gy[0][j][i] = fdb[r][0]; S.Gy[1][j][i] = fdb[r][1]; S.Gy[2][j][i] = fdb[r][2];
+        for (int r = 0; r < PER; ++r) {
+            const int idx = threadIdx.x + r * NT;
+            if (idx >= NCELL) continue;
+            int i, j;
+            block_cell<W - 4>(idx, H - 4, i, j);
+            i += 2; j += 2;
+            S.Gy[0][j][i] = fdb[r][0]; S.Gy[1][j][i] = fdb[r][1]; S.Gy[2][j][i] = fdb[r][2];
+        }
+        __syncthreads();
     }
-    __syncthreads();
     auto FDb = [&](int c) -> float (&)[H][W] { return S.Gy[c]; };
 
     // The reverse passes cover only what reaches the x-bar of the tile's
@@ -335,7 +342,8 @@ __device__ void stage_vjp_body(const GocCdklmParams& p, const StepConst& k, floa
         __syncthreads();
     }
     // 5. x slopes in reverse (three colours); their adjoints are complete
-    //    once the x faces are done
+    //    once the x faces are done, and each is cleared when read: the y
+    //    slopes' go to the same places
     constexpr int NXS = TX + 2, NYS = TY;       // x slopes of cells [T0X - 1, T1X + 1) on the tile's rows
 #pragma unroll 1
     for (int colour = 0; colour < 3; ++colour) {
@@ -348,13 +356,6 @@ __device__ void stage_vjp_body(const GocCdklmParams& p, const StepConst& k, floa
         }
         __syncthreads();
     }
-    // Fx is cleared again for the y-slope adjoints
-    for (int idx = threadIdx.x; idx < H * W; idx += NT) {
-        const int i = idx % W, j = idx / W;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) S.Fx[c][j][i] = 0.0f;
-    }
-    __syncthreads();
     // 6. y faces and y slopes in reverse
     if (!p.one_dimensional) {
         constexpr int NXG = TX, NYG = TY + 3;     // north faces of rows [T0Y - 2, T1Y + 1) on the tile's columns

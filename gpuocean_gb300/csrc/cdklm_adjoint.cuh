@@ -52,17 +52,19 @@ struct AdjSmem {
 // sign, else 0.
 __device__ __forceinline__ void minmod_raw_vjp(float b, float c, float f, float gb, float& bb, float& cb,
                                                float& fb) {
-    const float sb = copysignf(1.0f, b), sc = copysignf(1.0f, c), sf = copysignf(1.0f, f);
-    // no adjoint where the signs differ (branch-free: selects)
-    const float g = (sb == sc && sc == sf) ? gb : 0.0f;
     const float ab = fabsf(b), ac = fabsf(c), af = fabsf(f);
-    // inner min(|b|, |c|), outer min(., |f|)
-    const float wb1 = ab < ac ? 1.0f : (ab == ac ? 0.5f : 0.0f);
-    const float m1 = fminf(ab, ac);
-    const float wm = m1 < af ? 1.0f : (m1 == af ? 0.5f : 0.0f);
-    bb = b != 0.0f ? g * wb1 * wm : 0.0f;
-    cb = c != 0.0f ? g * (1.0f - wb1) * wm : 0.0f;
-    fb = f != 0.0f ? g * (1.0f - wm) : 0.0f;
+    // inner m = min(|b|, |c|), outer min(m, |f|)
+    const float m = fminf(ab, ac);
+    // no adjoint where the signs differ, nor where the minimum is 0: it is
+    // then |x| at x = 0 for all that it passes to (branch-free: selects)
+    const int signs = (__float_as_int(b) ^ __float_as_int(c)) | (__float_as_int(b) ^ __float_as_int(f));
+    const float g = (signs >= 0 && fminf(m, af) != 0.0f) ? gb : 0.0f;
+    const float wb = ab < ac ? 1.0f : (ab == ac ? 0.5f : 0.0f);
+    const float wm = m < af ? 1.0f : (m == af ? 0.5f : 0.0f);
+    const float gm = g * wm;
+    bb = gm * wb;
+    cb = gm - bb;
+    fb = g - gm;
 }
 
 __device__ __forceinline__ void minmod_slope_vjp(float l, float c, float r, float theta, float gs, float& lb,
@@ -124,14 +126,11 @@ __device__ __forceinline__ void cdklm_flux_vjp(const GocCdklmParams& p, const St
     const float hp = ep + H;
     const float hm = em + H;
     const bool wp = hp > p.depth_cutoff, wm = hm > p.depth_cutoff;
-    const float Fp0 = wp ? hp * up_ : 0.f;
-    const float Fp1 = wp ? hp * up_ * up_ + k.half_g * hp * hp : 0.f;
-    const float Fp2 = wp ? hp * up_ * vp_ : 0.f;
-    const float up = wp ? up_ : 0.f, cp = wp ? sqrtf(p.g * hp) : 0.f;
-    const float Fm0 = wm ? hm * um_ : 0.f;
-    const float Fm1 = wm ? hm * um_ * um_ + k.half_g * hm * hm : 0.f;
-    const float Fm2 = wm ? hm * um_ * vm_ : 0.f;
-    const float um = wm ? um_ : 0.f, cm = wm ? sqrtf(p.g * hm) : 0.f;
+    // a dry side has no depth and no velocity, hence no fluxes
+    const float hpw = wp ? hp : 0.f, up = wp ? up_ : 0.f;
+    const float Fp0 = hpw * up, Fp1 = Fp0 * up + k.half_g * hpw * hpw, Fp2 = Fp0 * vp_, cp = sqrtf(p.g * hpw);
+    const float hmw = wm ? hm : 0.f, um = wm ? um_ : 0.f;
+    const float Fm0 = hmw * um, Fm1 = Fm0 * um + k.half_g * hmw * hmw, Fm2 = Fm0 * vm_, cm = sqrtf(p.g * hmw);
     const float A = um + cm, B = up + cp, C = um - cm, D = up - cp;
     const float am = fminf(fminf(C, D), 0.0f);
     const float ap = fmaxf(fmaxf(A, B), 0.0f);
@@ -176,12 +175,12 @@ __device__ __forceinline__ void cdklm_flux_vjp(const GocCdklmParams& p, const St
     // the wet sides' terms (a dry side has none)
     float um_b = 0.f, up_b = 0.f;
     {
-        const float hmb_w = (cm > 0.0f ? cmb * 0.5f * p.g / cm : 0.0f) + Fm0b * um_ +
+        const float hmb_w = (cm > 0.0f ? __fdividef(cmb * k.half_g, cm) : 0.0f) + Fm0b * um_ +
                             Fm1b * (um_ * um_ + p.g * hm) + Fm2b * um_ * vm_;
         const float umb_w = umb_m + Fm0b * hm + Fm1b * 2.0f * hm * um_ + Fm2b * hm * vm_;
         const float vmb_w = Fm2b * hm * um_;
         if (wm) { hmb += hmb_w; um_b += umb_w; vm_b += vmb_w; }
-        const float hpb_w = (cp > 0.0f ? cpb * 0.5f * p.g / cp : 0.0f) + Fp0b * up_ +
+        const float hpb_w = (cp > 0.0f ? __fdividef(cpb * k.half_g, cp) : 0.0f) + Fp0b * up_ +
                             Fp1b * (up_ * up_ + p.g * hp) + Fp2b * up_ * vp_;
         const float upb_w = upb_m + Fp0b * hp + Fp1b * 2.0f * hp * up_ + Fp2b * hp * vp_;
         const float vpb_w = Fp2b * hp * up_;
@@ -218,16 +217,16 @@ __device__ __forceinline__ void friction_vjp(const GocCdklmParams& p, float dt, 
             hvb += q2;
         }
     } else {
-        const float u = hu / hsum, v = hv / hsum;
+        const float ih = 1.0f / hsum;
+        const float u = hu * ih, v = hv * ih;
         const float s = sqrtf(u * u + v * v);
-        const float C = dt * p.r * s / hsum;
-        const float sb = Cb * dt * p.r / hsum;
-        hsb += -Cb * C / hsum;
+        const float sb = Cb * dt * p.r * ih;
+        hsb += -sb * s * ih;
         if (s > 0.0f) {
-            const float ub = sb * u / s, vb = sb * v / s;
-            hub += ub / hsum;
-            hvb += vb / hsum;
-            hsb += -(ub * u + vb * v) / hsum;
+            const float w = __fdividef(sb, s) * ih;      // (u, v)-bar / (u h, v h)
+            hub += w * u;
+            hvb += w * v;
+            hsb += -w * (u * u + v * v);
         }
     }
 }
@@ -373,6 +372,7 @@ struct AdjTile {
         SM& S = A;
         const float g0 = Sxb(0)[j][i], g1 = Sxb(1)[j][i], g2 = Sxb(2)[j][i];
         if (g0 == 0.0f && g1 == 0.0f && g2 == 0.0f) return;
+        Sxb(0)[j][i] = 0.0f; Sxb(1)[j][i] = 0.0f; Sxb(2)[j][i] = 0.0f;   // the y slopes' place next
         const float th = p.theta;
         const int gx = T.x0 + i;
         const float eL = S.D[0][j][i - 1], eC = S.D[0][j][i], eR = S.D[0][j][i + 1];
