@@ -33,15 +33,19 @@ MODEL_TIME_STEP = 60.0
 NOISE_FACTOR = 8          # coarse grid every 8 cells
 NOISE_L_COARSE = 8.0      # SOAR length scale in coarse cells
 NOISE_STD = 0.003         # target std of the SOAR eta perturbation [m]
-# DRAM bytes (read + write) per member-cell-step of ensemble_rk2_kernel, from
-# one ncu capture of a 96-member C3 launch (221.0 MB read + 148.7 MB written
-# over 96 x 512 x 300 member-cell-steps, step built without FMA contraction);
-# traffic of a bench launch is scaled by its member-cells.
-NCU_DRAM_BYTES_PER_MEMBER_CELL = 369.7e6 / (96 * 512 * 300)
-# Warp instructions per member-cell-step of the same capture
-# (smsp__inst_executed.sum = 0.880e9): the step is bound by instruction issue,
-# whose ceiling is 4 warp instructions per cycle per SM.
-NCU_WARP_INST_PER_MEMBER_CELL = 0.880e9 / (96 * 512 * 300)
+# Per member-cell-step, from one ncu capture of a 96-member C3 launch
+# (96 x 512 x 300 member-cell-steps, step built without FMA contraction): DRAM
+# bytes (read + write) and warp instructions (smsp__inst_executed.sum).  The
+# step is bound by instruction issue, whose ceiling is 4 warp instructions per
+# cycle per SM.  The marching kernel runs where the autotuner picks its shape,
+# the tile kernel otherwise; what a bench launch moves and executes is scaled
+# by its member-cells.
+C3_SAMPLE = 96 * 512 * 300
+NCU_KERNELS = {
+    "ensemble_march_kernel": {"dram_bytes": 340.0e6 / C3_SAMPLE, "warp_inst": 0.4227e9 / C3_SAMPLE},
+    "ensemble_rk2_kernel": {"dram_bytes": 369.7e6 / C3_SAMPLE, "warp_inst": 0.880e9 / C3_SAMPLE},
+}
+MARCH_SHAPE = (56, 8)
 SM_COUNT = 152
 
 
@@ -466,13 +470,13 @@ def run_statistics(ens, sims, peak, peak_kind, n_positions=1000, repeats=10):
     return out
 
 
-def issue_roofline(member_cells, seconds, clk):
+def issue_roofline(kernel, member_cells, seconds, clk):
     """The fused step against its actual bound, instruction issue: warp
     instructions per launch (ncu count per member-cell-step x member-cells)
     per second, against 4 per cycle on each of the 152 SMs at the SM clock
     sampled during the timed region."""
     mhz = (clk or {}).get("sm_mhz") or 2070.0
-    achieved = NCU_WARP_INST_PER_MEMBER_CELL * member_cells / seconds / 1e9
+    achieved = NCU_KERNELS[kernel]["warp_inst"] * member_cells / seconds / 1e9
     peak = 4 * SM_COUNT * mhz * 1e6 / 1e9
     return {"achieved": achieved, "peak": peak, "unit": "G warp-instructions/s", "frac": achieved / peak,
             "source": "ncu smsp__inst_executed.sum of a 96-member launch, scaled per member-cell"}
@@ -880,7 +884,8 @@ def main():
         ens._ptrs = ens._current_ptrs()
     ens._sched_key = None
     avg_bytes = float(np.mean(bytes_k))
-    traffic = NCU_DRAM_BYTES_PER_MEMBER_CELL * float(np.mean(cells_k))
+    kernel = "ensemble_march_kernel" if tuple(ens.tile_shape) == MARCH_SHAPE else "ensemble_rk2_kernel"
+    traffic = NCU_KERNELS[kernel]["dram_bytes"] * float(np.mean(cells_k))
     avg_dur = float(np.mean(durations))
     achieved = avg_bytes / avg_dur / 1e9
     peak, peak_kind = measured_peaks()
@@ -1000,10 +1005,10 @@ def main():
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of a 96-member "
-                                           "launch, scaled per member-cell", "kernel": "ensemble_rk2_kernel",
+                                           "launch, scaled per member-cell", "kernel": kernel,
                          "peak_kind": peak_kind, "avg_launch_ms": 1000.0 * avg_dur,
                          "algorithmic_bytes_per_launch": avg_bytes,
-                         "issue": issue_roofline(float(np.mean(cells_k)), avg_dur, clk)},
+                         "issue": issue_roofline(kernel, float(np.mean(cells_k)), avg_dur, clk)},
             "e2e": e2e, "gpu_launches": launches, "clocks": clk, "cpu_baseline": cpu,
             "multilevel": multilevel, "adjoint": adjoint, "statistics": ens_stats, "kl_model_error": kl, "c2_ten_days": c2, "netcdf": netcdf, "open_boundaries": open_bc,
             "wall_s": wall,

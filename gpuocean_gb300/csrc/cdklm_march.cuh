@@ -29,10 +29,11 @@
 // rounding by rounding (a value that several faces or terms of the tile
 // kernel recompute is evaluated once here), so both give the same bits.
 //
-// Measured (256 members of 512 x 300, one step): 1.45 ms against 2.42 ms of
-// the tile kernel; per cell about 740 thread instructions against 1,870, 62 %
-// of the issue slots and 47 % of the FP32 pipe in use.  Eight strips per SM at
-// 128 registers a thread; six at 168 (1.72 ms) leave too few warps, ten at 96
+// Measured (256 members of 512 x 300, one step): 1.41 ms against 2.42 ms of
+// the tile kernel; 96 members 0.566 against 0.945 ms, 917 thread
+// instructions per cell (warp instructions x 32) against 1,910, 62 % of the
+// issue slots and 48 % of the FP32 pipe in use.  Eight strips per SM at 128
+// registers a thread; six at 168 (1.72 ms) leave too few warps, ten at 96
 // (1.75 ms) spill.
 #pragma once
 
@@ -555,10 +556,11 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
         const size_t og = (size_t)(r - 2) * G.pitch + gx0;
         unsigned s4 = march_stage(r);
         bool flip = false, lands = false;
-        hist <<= 1;
+        const bool ghost_row = !py && (unsigned)(r - 2) >= (unsigned)ny;     // beyond a wall
+        hist = hist << 1 | (unsigned)general;
         if (second) {
             // input row Q*, wall mirrors folded back, and Q^n of the output row
-            if (__builtin_expect(!py && (r < 2 || r >= ny + 2), 0)) {
+            if (__builtin_expect(ghost_row, 0)) {
                 s4 = march_stage(r < 2 ? 3 - r : 2 * ny + 3 - r);
                 flip = true;
             }
@@ -580,7 +582,7 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
             if (r + 2 <= a1) issue(r + 2);
             cp_async_commit();
             cp_async_wait<2>();
-            if (__builtin_expect(!py && (r < 2 || r >= ny + 2), 0)) {
+            if (__builtin_expect(ghost_row, 0)) {
                 flip = true;
                 float2& f = at(FC, oU);
                 f = G.F ? pr(-f.x, -f.y) : pr(-f0);
@@ -648,7 +650,7 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
             at(HC, oC) = mul2(c.quarter, plain_add(plain_add(AA, Bp), B));
             if (lane == 0) S.land[r & (kMarchRing - 1)] = (int)(hist & 1u);
         }
-        slow = slow || general || (hist & 7u) != 0 || (!py && r == ny + 3);
+        slow = slow || (hist & 7u) != 0 || (ghost_row && r == ny + 3);
         MarchRhs R;
         if (__builtin_expect(!slow, 1)) {
             // ---- y slopes of row C ----
