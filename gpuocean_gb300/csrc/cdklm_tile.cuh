@@ -1199,7 +1199,7 @@ __device__ __forceinline__ bool cdklm_strip_tile(const GocCdklmParams& p, const 
 }
 
 template <int TX, int TY, int NSTAGE, int NT, bool CONST_F, bool SIMPLE_FORCING, bool ANGLE = false>
-__global__ void __launch_bounds__(NT, NT > 256 ? 1 : ANGLE ? 2 : 3)
+__global__ void __launch_bounds__(NT, NT == 512 ? 2 : NT > 256 ? 1 : ANGLE ? 2 : 3)
 cdklm_tile_kernel(const GocCdklmParams p, const StepConst k, float dt, int rk_step,
                   const float* __restrict__ e_in, const float* __restrict__ hu_in,
                   const float* __restrict__ hv_in, float* e_out, float* hu_out, float* hv_out,

@@ -1,7 +1,7 @@
-"""Steps of small grids: the tile shapes and thread counts that grids with few
-tiles take give the bits of the engine's tiles (32 x 16 cells, 256 threads).
-The sizes sit on both sides of the two limits (38 and 152 tiles) and at ragged
-edges of the 16 x 8 tiles."""
+"""Steps of small and large grids: the tile shapes and thread counts that grids
+with few or many tiles take give the bits of the engine's tiles (32 x 16 cells,
+256 threads).  The sizes sit on both sides of the limits (38 and 152 tiles, 912
+tiles of 32 x 32) and at ragged edges of the 16 x 8 and 32 x 32 tiles."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
     (1, 1, (1, 1, 1, 1), 0.0, 0.0), (5, 4, (2, 2, 2, 2), 0.0, 0.0), (16, 8, (1, 2, 1, 2), 2e-11, 0.0),
     (17, 9, (1, 1, 1, 1), 0.0, 1e-3), (64, 64, (1, 1, 1, 1), 2e-11, 0.0), (608, 32, (1, 2, 1, 2), 0.0, 0.0),
     (609, 32, (1, 2, 1, 2), 2e-11, 0.0), (255, 257, (2, 1, 2, 1), 0.0, 1e-3), (2432, 32, (1, 2, 1, 2), 2e-11, 0.0),
-    (2433, 32, (1, 1, 1, 1), 0.0, 0.0)])
+    (2433, 32, (1, 1, 1, 1), 0.0, 0.0), (1216, 768, (1, 1, 1, 1), 2e-11, 1e-3), (1185, 737, (2, 2, 2, 2), 0.0, 0.0),
+    (1184, 768, (1, 2, 1, 2), 2e-11, 0.0), (33, 29153, (1, 1, 1, 1), 0.0, 0.0)])
 def test_small_grids_step_like_tiles(gpu_ctx, nx, ny, bc, beta, r):
     from gpuocean_gb300.SWEsimulators.CDKLM16 import CDKLM16
     from gpuocean_gb300.ensembles.BatchedEnsemble import BatchedEnsemble
