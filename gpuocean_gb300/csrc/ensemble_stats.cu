@@ -120,12 +120,16 @@ __device__ __forceinline__ void pair_values(const float2* v, float eps, float2* 
 }
 
 // s += a with what the rounding lost kept in c (Kahan): the members' sums
-// would else run longer than those of a slice did.
-__device__ __forceinline__ void add_to(float2& s, float2& c, float2 a) {
-    const float2 y = make_float2(__fsub_rn(a.x, c.x), __fsub_rn(a.y, c.y));
-    const float2 t = make_float2(__fadd_rn(s.x, y.x), __fadd_rn(s.y, y.y));
-    c = make_float2(__fsub_rn(__fsub_rn(t.x, s.x), y.x), __fsub_rn(__fsub_rn(t.y, s.y), y.y));
+// would else run longer than those of a slice did.  A sum that is no longer
+// finite has lost nothing: inf - inf would make it NaN at the next member.
+__device__ __forceinline__ void add_to(float& s, float& c, float a) {
+    const float y = __fsub_rn(a, c), t = __fadd_rn(s, y);
+    c = fabsf(t) < INFINITY ? __fsub_rn(__fsub_rn(t, s), y) : 0.0f;
     s = t;
+}
+__device__ __forceinline__ void add_to(float2& s, float2& c, float2 a) {
+    add_to(s.x, c.x, a.x);
+    add_to(s.y, c.y, a.y);
 }
 
 // One slice of the members: shifted sums s1 = sum(x - K), s2 = sum((x - K)^2)
