@@ -635,9 +635,10 @@ class BatchedEnsemble:
                 _lib.call("goc_ensemble_set_block_noise", self._handle, None, -1)
         if noise == "block" and not fused:
             # the members that take model error in this block; SOAR draws new
-            # normals for every member, as ahead of a fused step
+            # normals for every member, as ahead of a fused step, and like
+            # that none in a block without steps
             if self._noise_kind == "soar":
-                if self._rng_seed is not None:
+                if self._rng_seed is not None and nsub > 0:
                     _lib.call("goc_noise_batch_generate", self._noise, self._handle, -1, self.stream.handle)
                 self._noise_launch(-2, update_random_field=False)
             else:
