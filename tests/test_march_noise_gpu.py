@@ -38,6 +38,31 @@ def _same(a, b):
     return len(a) == len(b) and all(np.array_equal(x, y) for x, y in zip(a, b))
 
 
+@pytest.mark.parametrize("factor", [1, 3, 7])
+@pytest.mark.parametrize("rng_seed", [None, 5])
+@pytest.mark.parametrize("cadence", ["block", "step"])
+def test_noise_is_the_same_on_every_shape(gpu_ctx, factor, rng_seed, cadence):
+    """Both cadences, injected and drawn normals, members without model error,
+    blocks of unequal length, an idle member, drifters, factors on both sides
+    of the row transfer's."""
+    from gpuocean_gb300.ensembles.BatchedEnsemble import BatchedEnsemble
+    first = None
+    for shape in BatchedEnsemble.tile_shapes():
+        ens, sims = _engine(gpu_ctx, shape, factor, rng_seed)
+        assert ens._marches() == (shape == (56, 8))
+        ens.step(300.0, True, noise_cadence=cadence)
+        ens.step(300.0, [True, False, True, True], noise_cadence=cadence)
+        ens.step(200.0, True, noise_cadence=cadence, members=[0, 2, 3])
+        ens.step(300.0, False)
+        ens.step(300.0, True, noise_cadence=cadence)
+        assert len({s.num_iterations for s in sims}) > 1
+        got = _results(ens, sims)
+        ens.release()
+        if first is None:
+            first = got
+        assert _same(got, first), shape
+
+
 @pytest.mark.parametrize("use_graph", [False, True])
 @pytest.mark.parametrize("shape", [(32, 16), (56, 8)])
 def test_blocks_without_steps_draw_nothing(gpu_ctx, shape, use_graph):
