@@ -142,12 +142,12 @@ __device__ __forceinline__ void add_to(float2& s, float2& c, float2 a) {
 // thread, four members in flight and six slices took 92 us with their sum.
 template <int Q, bool WIDE>
 __global__ void __launch_bounds__(kMX * kMY) moments_kernel(const GocMemberDesc* __restrict__ mem, int first, int n,
-                                                            int per_slice, int nx, int ny, float eps, int ddof,
-                                                            float* __restrict__ mean, float* __restrict__ var,
-                                                            float* __restrict__ part) {
+                                                            int per_slice, int nx, int ny, int first_row, float eps,
+                                                            int ddof, float* __restrict__ mean,
+                                                            float* __restrict__ var, float* __restrict__ part) {
     constexpr int P = Q == 0 ? 3 : 2, A = Q == 0 ? 3 : 4;
     __shared__ MomentSrc s_src[kMChunk];
-    const int x = 2 * (blockIdx.x * kMX + threadIdx.x), y = blockIdx.y * kMY + threadIdx.y;
+    const int x = 2 * (blockIdx.x * kMX + threadIdx.x), y = first_row + blockIdx.y * kMY + threadIdx.y;
     const int t = threadIdx.y * kMX + threadIdx.x;
     const bool inside = x < nx && y < ny;
     const int m0 = blockIdx.z * per_slice, m1 = min(n, m0 + per_slice);
@@ -402,9 +402,15 @@ extern "C" int goc_ensemble_moments(void* ensemble, int first_member, int n_memb
     const GocMemberDesc* dm = ensemble_device_members(ensemble);
     const auto kernel = quantity == 0 ? (wide ? moments_kernel<0, true> : moments_kernel<0, false>)
                                       : (wide ? moments_kernel<1, true> : moments_kernel<1, false>);
-    kernel<<<grd, blk, 0, st>>>(dm, first_member, n_members, per_slice, nx, ny, desing_eps, ddof, mean, var, part);
-    count_launch();
-    int rc = check_launch("moments_kernel");
+    // one launch, or several on grids of more rows than 65535 blocks take
+    int rc = GOC_OK;
+    for (int row = 0; row < ny && !rc; row += 65535 * kMY) {
+        grd.y = std::min(65535, (ny - row + kMY - 1) / kMY);
+        kernel<<<grd, blk, 0, st>>>(dm, first_member, n_members, per_slice, nx, ny, row, desing_eps, ddof, mean, var,
+                                    part);
+        count_launch();
+        rc = check_launch("moments_kernel");
+    }
     if (rc || slices == 1) return rc;
     grd = dim3((nx + kMX - 1) / kMX, (ny + kMY - 1) / kMY);
     if (quantity == 0)

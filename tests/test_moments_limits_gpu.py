@@ -2,7 +2,8 @@
 import numpy as np
 import pytest
 
-from test_ensemble_stats_gpu import _stepped
+from test_ensemble_stats_gpu import _close, _stepped
+from test_march_gpu import WALLS, _sim
 
 pytestmark = pytest.mark.gpu
 
@@ -33,4 +34,18 @@ def test_members_that_are_not_finite(gpu_ctx, n, quantity):
         for j, i in spots:
             a[q, j - 2, i - 2] = b[q, j - 2, i - 2] = 0.0
         assert np.array_equal(a, b)
+    ens.release()
+
+
+def test_moments_of_a_tall_grid(gpu_ctx):
+    """More rows than a launch has blocks in y when a block takes four."""
+    from gpuocean_gb300.ensembles.BatchedEnsemble import BatchedEnsemble
+    nx, ny = 3, 262149
+    sims = [_sim(gpu_ctx, nx, ny, WALLS, m) for m in range(3)]
+    ens = BatchedEnsemble(sims, autotune=False)
+    mean, var = ens.moments()
+    x = np.stack([np.stack([np.asarray(np.ma.getdata(a))[2:-2, 2:-2] for a in s.download()]) for s in sims])
+    x = x.astype(np.float64)
+    for q in range(3):      # the bars of the other moments tests
+        assert _close(mean[q], x[:, q].mean(axis=0), 2e-6) and _close(var[q], x[:, q].var(axis=0), 1e-5)
     ens.release()
