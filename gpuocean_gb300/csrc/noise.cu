@@ -298,8 +298,11 @@ __device__ void kl_perturb_tile(const GocKLDesc& d, const OceanRef& o, float sca
 }
 
 __global__ void kl_table_kernel(GocKLDesc d, int nx, int ny) {
-    kl_table_entry(d, KLRoll{d.roll_x_sin, d.roll_y_sin, d.roll_x_cos, d.roll_y_cos}, nx, ny, blockIdx.z,
-                   blockIdx.y * kTableThreads + threadIdx.x, blockIdx.x);
+    // the blocks of an entry's rows are neighbours in x: neither the columns nor
+    // the basis rows end at the 65535 blocks of grid.y
+    const int rows = kl_count_y(d);
+    kl_table_entry(d, KLRoll{d.roll_x_sin, d.roll_y_sin, d.roll_x_cos, d.roll_y_cos}, nx, ny, blockIdx.y,
+                   (int)blockIdx.x / rows * kTableThreads + threadIdx.x, (int)blockIdx.x % rows);
 }
 
 __global__ void __launch_bounds__(kKX * kKT, 4) kl_perturb_kernel(GocKLDesc d, OceanRef o, float scale, int eta_only) {
@@ -607,7 +610,7 @@ extern "C" int goc_kl_perturb(const GocKLDesc* kl, int nx, int ny, float dx, flo
     }
     cudaStream_t st = as_stream(stream);
     const int ntab = std::max(nx, ny) + 2;
-    kl_table_kernel<<<dim3(kl_count_y(*kl), (ntab + kTableThreads - 1) / kTableThreads, 2), kTableThreads, 0, st>>>(
+    kl_table_kernel<<<dim3(kl_count_y(*kl) * ((ntab + kTableThreads - 1) / kTableThreads), 2), kTableThreads, 0, st>>>(
         *kl, nx, ny);
     count_launch();
     if ((rc = check_launch("kl_table_kernel"))) return rc;
