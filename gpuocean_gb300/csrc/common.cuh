@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+
 #include "../../include/gpuocean_gb300.h"
 
 namespace goc {
@@ -27,6 +29,22 @@ const GocMemberDesc* ensemble_device_members(void* ensemble);
 const int* ensemble_device_nsub(void* ensemble);
 // per member the block's step count if the member takes model error, else 0
 const int* ensemble_device_noise_steps(void* ensemble);
+
+// The slices' sums of an engine's goc_ensemble_moments (ensemble_stats.cu),
+// allocated with the engine.  A call holds in_use from take to give, so calls
+// of several threads do not share them; on the device a call waits for the last
+// one's event, whichever stream that ran on.
+struct MomentScratch {
+    std::mutex in_use;
+    float* sums = nullptr;
+    cudaEvent_t done = nullptr;
+    bool captured = false;
+    cudaError_t create(const GocMemberDesc* members, int n_members);
+    int take(cudaStream_t st);
+    int give(cudaStream_t st);
+    void release();
+};
+MomentScratch* ensemble_moment_scratch(void* ensemble);
 
 // Device table of the members' SOAR descriptors of a noise batch handle
 // (noise.cu); n_members receives the batch's member count.

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(256) ensemble_dt_final_kernel(const float* __r
 }
 
 static void free_ensemble(Ensemble* e) {
+    e->moment_scratch.release();
     cudaFree(e->d_members);
     cudaFree(e->d_tiles);
     cudaFree(e->d_march);
@@ -247,6 +248,8 @@ const GocMemberDesc* ensemble_device_members(void* ensemble) { return static_cas
 const int* ensemble_device_nsub(void* ensemble) { return static_cast<Ensemble*>(ensemble)->d_nsub; }
 
 const int* ensemble_device_noise_steps(void* ensemble) { return static_cast<Ensemble*>(ensemble)->d_nsub_noise; }
+
+MomentScratch* ensemble_moment_scratch(void* ensemble) { return &static_cast<Ensemble*>(ensemble)->moment_scratch; }
 
 static int shape_configure(const Ensemble* e, int* grid) {
     if (e->shape == kMarchShape && e->can_march) {
@@ -518,6 +521,7 @@ extern "C" int goc_ensemble_create(const GocMemberDesc* members, int n_members, 
     if (err == cudaSuccess) err = cudaMemset(e->d_dt, 0, sizeof(float) * (size_t)n_members * max_substeps);
     if (err == cudaSuccess) err = cudaMalloc(&e->d_queue, sizeof(int));
     if (err == cudaSuccess) err = cudaMemset(e->d_queue, 0, sizeof(int));
+    if (err == cudaSuccess) err = e->moment_scratch.create(members, n_members);
     if (err != cudaSuccess) {
         free_ensemble(e);
         return set_error(GOC_ERR_CUDA, "goc_ensemble_create: %s", cudaGetErrorString(err));

@@ -102,6 +102,7 @@ struct Ensemble {
     int4* d_march = nullptr;
     int n_march = 0;
     bool can_march = false;
+    MomentScratch moment_scratch;
     int tile_shape() const { return shape == kMarchShape ? 0 : shape; }
 };
 

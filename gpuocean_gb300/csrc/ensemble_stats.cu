@@ -9,6 +9,7 @@
 // pass over HBM gives mean and variance of a member group, and the multi-level
 // estimator is assembled on the finest grid in one more launch.
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -262,6 +263,57 @@ __global__ void moments_finish_kernel(const GocMemberDesc* __restrict__ mem, int
     }
 }
 
+// Slices of n members of an nx x ny grid, until each SM has two blocks: fewer
+// leave too few loads in flight, more only add sums to write and read (96
+// members of 512 x 300, velocities: 39 us in one slice, 46 in two, 49 in three).
+static int moment_slices(int nx, int ny, int n, int* per_slice) {
+    const long long blocks = (long long)((nx + 2 * kMX - 1) / (2 * kMX)) * ((ny + kMY - 1) / kMY);
+    const int most = (int)std::min<long long>(std::max<long long>(1, (152LL * kMBlocks + blocks - 1) / blocks),
+                                              std::max(1, n / 16));
+    *per_slice = (n + std::min(most, 65535) - 1) / std::min(most, 65535);
+    return (n + *per_slice - 1) / *per_slice;
+}
+
+static int scratch_error(cudaError_t err) {
+    return err == cudaSuccess ? GOC_OK
+                              : set_error(GOC_ERR_CUDA, "goc_ensemble_moments: scratch: %s", cudaGetErrorString(err));
+}
+
+cudaError_t MomentScratch::create(const GocMemberDesc* members, int n_members) {
+    // room for any group of members: of n members, at most n / 16 slices
+    size_t floats = 0;
+    for (int m = 0; m < n_members; ++m) {
+        const GocCdklmParams& p = members[m].p;
+        const long long blocks = (long long)((p.nx + 2 * kMX - 1) / (2 * kMX)) * ((p.ny + kMY - 1) / kMY);
+        const long long most = std::min<long long>((152LL * kMBlocks + blocks - 1) / blocks, n_members / 16);
+        if (most > 1) floats = std::max(floats, (size_t)most * 6 * p.nx * p.ny);
+    }
+    if (floats == 0) return cudaSuccess;
+    const cudaError_t err = cudaMalloc(&sums, floats * sizeof(float));
+    return err != cudaSuccess ? err : cudaEventCreateWithFlags(&done, cudaEventDisableTiming);
+}
+
+// While calls on `st` are captured into a graph, the graph orders its launches,
+// and events of other streams are out of its reach.
+int MomentScratch::take(cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaError_t err = cudaStreamIsCapturing(st, &status);
+    captured = status != cudaStreamCaptureStatusNone;
+    if (err == cudaSuccess && !captured) err = cudaStreamWaitEvent(st, done, 0);
+    return scratch_error(err);
+}
+
+int MomentScratch::give(cudaStream_t st) {
+    return scratch_error(captured ? cudaSuccess : cudaEventRecord(done, st));
+}
+
+void MomentScratch::release() {
+    cudaFree(sums);
+    if (done) cudaEventDestroy(done);
+    sums = nullptr;
+    done = nullptr;
+}
+
 // ---------------------------------------------------------------------------
 // multi-level estimator (E/MultiLevelOceanEnsemble.py:258-267)
 // ---------------------------------------------------------------------------
@@ -296,13 +348,6 @@ __global__ void ml_combine_kernel(MLLevels L, double* __restrict__ out) {
     }
     out[((size_t)p * NY + y) * NX + x] = est;
 }
-
-// Scratch for the per-slice sums, owned by the library (one per process).
-struct StatsScratch {
-    float* ptr = nullptr;
-    size_t bytes = 0;
-};
-StatsScratch g_scratch;
 
 }  // namespace goc
 
@@ -370,33 +415,18 @@ extern "C" int goc_ensemble_moments(void* ensemble, int first_member, int n_memb
         for (int set = 0; set < 2; ++set) bits |= (uintptr_t)d.eta[set] | (uintptr_t)d.hu[set] | (uintptr_t)d.hv[set];
         wide = wide && (bits & 7u) == 0;
     }
-    const int P = quantity == 0 ? 3 : 2;
-    const size_t cells = (size_t)nx * ny;
     dim3 blk(kMX, kMY), grd((nx + 2 * kMX - 1) / (2 * kMX), (ny + kMY - 1) / kMY);
-    // slices of the members until each SM has two blocks: fewer leave too few
-    // loads in flight, more only add sums to write and read (96 members of
-    // 512 x 300, velocities: 39 us in one slice, 46 in two, 49 in three)
-    const long long blocks = (long long)grd.x * grd.y;
-    int slices = (int)std::min<long long>(std::max<long long>(1, (152LL * kMBlocks + blocks - 1) / blocks),
-                                          std::max(1, n_members / 16));
-    slices = std::min(slices, 65535);
-    const int per_slice = (n_members + slices - 1) / slices;
-    slices = (n_members + per_slice - 1) / per_slice;
-    cudaStream_t st = as_stream(stream);
+    int per_slice = 0;
+    const int slices = moment_slices(nx, ny, n_members, &per_slice);
+    const cudaStream_t st = as_stream(stream);
     float* part = nullptr;
+    // the slices' sums pass through the engine's scratch, one call at a time
+    MomentScratch& scratch = *ensemble_moment_scratch(ensemble);
+    std::unique_lock<std::mutex> lock(scratch.in_use, std::defer_lock);
     if (slices > 1) {
-        const size_t need = (size_t)slices * 2 * P * cells * sizeof(float);
-        if (g_scratch.bytes < need) {
-            cudaError_t err = cudaStreamSynchronize(st);
-            if (err == cudaSuccess) err = cudaFree(g_scratch.ptr);
-            g_scratch.ptr = nullptr;
-            g_scratch.bytes = 0;
-            if (err == cudaSuccess) err = cudaMalloc(&g_scratch.ptr, need);
-            if (err != cudaSuccess)
-                return set_error(GOC_ERR_CUDA, "goc_ensemble_moments: scratch: %s", cudaGetErrorString(err));
-            g_scratch.bytes = need;
-        }
-        part = g_scratch.ptr;
+        lock.lock();
+        if (const int rc = scratch.take(st)) return rc;
+        part = scratch.sums;
     }
     grd.z = slices;
     const GocMemberDesc* dm = ensemble_device_members(ensemble);
@@ -420,7 +450,8 @@ extern "C" int goc_ensemble_moments(void* ensemble, int first_member, int n_memb
         moments_finish_kernel<1><<<grd, blk, 0, st>>>(dm, first_member, n_members, slices, nx, ny, desing_eps, ddof,
                                                       part, mean, var);
     count_launch();
-    return check_launch("moments_finish_kernel");
+    rc = check_launch("moments_finish_kernel");
+    return rc ? rc : scratch.give(st);
 }
 
 extern "C" int goc_ml_combine(int n_levels, const float* const* fine, const float* const* coarse, const int* nx,
