@@ -14,9 +14,9 @@ different numbers of steps; a member whose block is done idles.
 """
 from __future__ import annotations
 
-import collections
 import ctypes
 import operator
+import threading
 
 import numpy as np
 
@@ -28,6 +28,55 @@ from ..utils import Common
 _AUTOTUNE_CACHE = {}
 # a simulator's current state buffer, by which the engine sees that members were swapped or replaced
 _state_address = operator.attrgetter("gpu_data.h0.data.ptr")
+
+
+class _MomentBuffers:
+    """The device buffers of moments() between calls, two at most for all
+    engines of the process: allocating and freeing them took 170 of 390 us (96
+    members of 512 x 300), and an engine's first call pays that again where
+    each engine keeps its own.  A buffer belongs to one call from take to put,
+    which comes after the call's stream was waited for, so engines, threads
+    and streams share the pool; a call that finds it empty takes new buffers.
+    The last engine to go frees them."""
+
+    def __init__(self):
+        self._lock = threading.Lock()
+        self._free = []
+        self._engines = 0
+
+    def take(self, nbytes):
+        """A device buffer of at least nbytes; kept ones that are too small
+        make room for it."""
+        with self._lock:
+            fits = next((b for b in self._free if b.nbytes >= nbytes), None)
+            small = [] if fits else self._free
+            self._free = [b for b in self._free if b is not fits] if fits else []
+        for b in small:
+            b.free()
+        return fits or Common.DevicePtr(nbytes)
+
+    def put(self, buf):
+        with self._lock:
+            keep = self._engines > 0 and len(self._free) < 2
+            if keep:
+                self._free.append(buf)
+        if not keep:
+            buf.free()
+
+    def open(self):
+        with self._lock:
+            self._engines += 1
+
+    def close(self):
+        with self._lock:
+            self._engines -= 1
+            gone = [] if self._engines else self._free
+            self._free = self._free if self._engines else []
+        for b in gone:
+            b.free()
+
+
+_MOMENT_BUFFERS = _MomentBuffers()
 
 
 class GocMemberDesc(ctypes.Structure):
@@ -111,7 +160,6 @@ class BatchedEnsemble:
         self._handle = None
         self._noise = None
         self._noise_kind = None
-        self._moment_bufs = collections.deque()     # device buffers of moments() between calls, two at most
         self._noises = None
         self._noise_sources = None
         self._rng_seed = None
@@ -125,6 +173,8 @@ class BatchedEnsemble:
             self._dedupe_coriolis()
         self._orig_streams = []
         self._adopt_streams(self.sims)
+        _MOMENT_BUFFERS.open()
+        self._open = True
         self._build()
         if autotune:
             self.autotune()
@@ -320,11 +370,11 @@ class BatchedEnsemble:
         """Free the device handles and give the members their own streams back."""
         self._release_handles()
         self._restore_streams()
+        if self.__dict__.pop("_open", False):
+            _MOMENT_BUFFERS.close()
 
     def _release_handles(self):
         self.release_noise()
-        while getattr(self, "_moment_bufs", None):
-            self._moment_bufs.popleft().free()
         for name in ("_obs_pos", "_obs_out", "_drift_gather", "_obs_scatter"):
             buf = getattr(self, name, None)
             if buf is not None:
@@ -848,9 +898,7 @@ class BatchedEnsemble:
         s0 = self.sims[first]
         planes = 3 if quantity == "state" else 2
         nbytes = 4 * planes * int(s0.nx) * int(s0.ny)
-        # allocating and freeing the two buffers took 170 of 390 us (96 members
-        # of 512 x 300): those that are not handed out are kept for later calls
-        new = self._take_moment_buffer if download else Common.DevicePtr
+        new = _MOMENT_BUFFERS.take if download else Common.DevicePtr
         bm = new(nbytes) if mean else None
         bv = new(nbytes) if var else None
         eps = 0.0 if desingularise is None else float(desingularise)
@@ -864,27 +912,8 @@ class BatchedEnsemble:
         out = tuple(None if b is None else self._download(b, shape) for b in (bm, bv))
         for b in (bm, bv):
             if b is not None:
-                self._put_moment_buffer(b)
+                _MOMENT_BUFFERS.put(b)
         return out
-
-    def _take_moment_buffer(self, nbytes):
-        """A device buffer of at least nbytes: one put back by an earlier call
-        if it is large enough.  A call that runs meanwhile on another thread
-        finds it gone and takes its own."""
-        while True:
-            try:
-                buf = self._moment_bufs.popleft()
-            except IndexError:
-                return Common.DevicePtr(nbytes)
-            if buf.nbytes >= nbytes:
-                return buf
-            buf.free()
-
-    def _put_moment_buffer(self, buf):
-        if len(self._moment_bufs) < 2:
-            self._moment_bufs.append(buf)
-        else:
-            buf.free()
 
     def max_dt(self):
         """Per member the CFL limit 0.25 min(dx / |u +- c|, dy / |v +- c|)
