@@ -152,6 +152,7 @@ class CDKLM16(Simulator):
         # RK stages run one launch each (goc_cdklm_stage) with the ghost fill
         # between them, as the reference steps
         self.angle_varies = angle.size != 1
+        self.angle_turned = bool(np.any(angle != 0.0))
         self.angle_arr = Common.CUDAArray2D(self.gpu_stream, angle.shape[1], angle.shape[0], 0, 0, angle)
         # a spatially varying texture is evaluated once per cell centre
         self.coriolis_cell = None

@@ -156,6 +156,7 @@ SIGNATURES = {
     "goc_ensemble_set_tile_shape": (c_int, [c_void_p, c_int]),
     "goc_ensemble_get_tile_shape": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
     "goc_ensemble_marches": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
+    "goc_ensemble_can_march": (c_int, [c_void_p, ctypes.POINTER(c_int)]),
     "goc_ensemble_get_member": (c_int, [c_void_p, c_int, c_void_p, c_void_p]),
     "goc_ensemble_max_dt": (c_int, [c_void_p, c_void_p, c_void_p]),
     "goc_ensemble_set_drifters": (c_int, [c_void_p, c_void_p, ctypes.POINTER(c_int), c_float, c_void_p]),

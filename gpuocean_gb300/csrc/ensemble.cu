@@ -761,6 +761,12 @@ extern "C" int goc_ensemble_marches(void* ensemble, int* marches) {
     return GOC_OK;
 }
 
+extern "C" int goc_ensemble_can_march(void* ensemble, int* can_march) {
+    if (!ensemble || !can_march) return set_error(GOC_ERR_ARG, "goc_ensemble_can_march: null argument");
+    *can_march = static_cast<Ensemble*>(ensemble)->can_march;
+    return GOC_OK;
+}
+
 extern "C" int goc_ensemble_end_block(void* ensemble, int n_launched, void* stream) {
     if (!ensemble) return set_error(GOC_ERR_ARG, "goc_ensemble_end_block: null handle");
     Ensemble* e = static_cast<Ensemble*>(ensemble);

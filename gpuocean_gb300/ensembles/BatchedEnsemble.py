@@ -26,6 +26,8 @@ from ..utils import Common
 
 # member grid signature -> index of the fastest tile shape (per process)
 _AUTOTUNE_CACHE = {}
+# the tile shape that stands for the marching kernel
+MARCH_SHAPE = (56, 8)
 # a simulator's current state buffer, by which the engine sees that members were swapped or replaced
 _state_address = operator.attrgetter("gpu_data.h0.data.ptr")
 
@@ -446,26 +448,42 @@ class BatchedEnsemble:
             _lib.load().goc_graph_destroy(g[0])
         self._graphs = {}
 
+    def _can_march(self):
+        """Whether the marching kernel takes every member."""
+        out = ctypes.c_int()
+        _lib.call("goc_ensemble_can_march", self._handle, ctypes.byref(out))
+        return bool(out.value)
+
     def _grid_signature(self):
+        """What the fastest tile shape depends on: the grids, and of each
+        member what sets a kernel's path (walls, land, a turned north vector,
+        one dimension) and its lookups (Coriolis table, forcing textures)."""
         sizes = {}
-        for s in self.sims:
+        flags = set()
+        for s, d in zip(self.sims, self._descs_host):
             key = (int(s.nx), int(s.ny))
             sizes[key] = sizes.get(key, 0) + 1
-        flags = tuple(sorted({(s.coriolis_cell is None, int(s.boundary_conditions.east)) for s in self.sims}))
-        return (tuple(sorted(sizes.items())), flags)
+            p = d.p
+            textures = p.wind_x_nx * p.wind_x_ny * p.wind_y_nx * p.wind_y_ny * p.atm_p_nx * p.atm_p_ny > 1
+            flags.add((s.coriolis_cell is None, int(p.bc_east), int(p.bc_north), bool(s.bathymetry.use_mask),
+                       s.angle_turned, bool(p.one_dimensional), textures))
+        return (tuple(sorted(sizes.items())), tuple(sorted(flags)))
 
     def autotune(self, repeats=5, candidates=None):
         """Time the persistent RK2 launch of every tile shape on this
         ensemble and keep the fastest.  Each timed launch is RK2 step 0 of a
         one-step schedule: it reads buffer set 0 (the current state) and
         writes set 1, so the members' state is left as it was.  Results are
-        cached per process by member grid sizes."""
+        cached per process by what they depend on (_grid_signature).  By
+        default every shape is a candidate that the members can run."""
         sig = self._grid_signature()
         best = _AUTOTUNE_CACHE.get(sig)
         if best is None:
             self._after_members()
             shapes = self.tile_shapes()
             idx = list(range(len(shapes))) if candidates is None else list(candidates)
+            if candidates is None and not self._can_march():
+                idx.remove(shapes.index(MARCH_SHAPE))   # it would time 32 x 16 a second time
             n = len(self.sims)
             table = np.zeros((n, self.max_substeps), dtype=np.float32)
             table[:, 0] = [np.float32(s.dt) for s in self.sims]

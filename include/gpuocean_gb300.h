@@ -532,6 +532,12 @@ int goc_ensemble_get_tile_shape(void* ensemble, int* index);
  */
 int goc_ensemble_marches(void* ensemble, int* marches);
 
+/* Whether the marching kernel takes every member of the ensemble, whichever
+ * tile shape is set.  With its shape set on an ensemble that it does not take,
+ * steps run the first tile shape.
+ */
+int goc_ensemble_can_march(void* ensemble, int* can_march);
+
 /* Close a block of `n_launched` substeps: advects the drifters of the last
  * step of members that ran all of them, then makes buffer set 0 the current
  * state again (swaps members whose block had an odd number of steps).
