@@ -42,7 +42,8 @@ class _MomentBuffers:
     The last engine to go frees them."""
 
     def __init__(self):
-        self._lock = threading.Lock()
+        # reentrant: a collection inside a call may release an engine
+        self._lock = threading.RLock()
         self._free = []
         self._engines = 0
 
