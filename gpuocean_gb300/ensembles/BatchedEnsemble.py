@@ -445,6 +445,7 @@ class BatchedEnsemble:
     def set_tile_shape(self, index):
         _lib.call("goc_ensemble_set_tile_shape", self._handle, int(index))
         self._shape_index = int(index)
+        self._make_copies()
         for g in self._graphs.values():
             _lib.load().goc_graph_destroy(g[0])
         self._graphs = {}
@@ -598,10 +599,7 @@ class BatchedEnsemble:
             _lib.call("goc_noise_batch_create", self._handle, descs, ctypes.byref(h))
             self._noise, self._noise_kind = h.value, "soar"
             self._noise_descs = descs
-            # the unperturbed copies that fused model error at the block
-            # cadence needs are allocated here, outside any graph capture
-            _lib.call("goc_ensemble_set_block_noise", self._handle, self._noise, 0)
-            _lib.call("goc_ensemble_set_block_noise", self._handle, None, -1)
+            self._make_copies()
             if rng_seed is not None:
                 _lib.call("goc_noise_batch_seed", self._noise, ctypes.c_ulonglong(int(rng_seed)), self.stream.handle)
         self._noises = noises
@@ -610,6 +608,14 @@ class BatchedEnsemble:
         for g in self._graphs.values():
             _lib.load().goc_graph_destroy(g[0])
         self._graphs = {}
+
+    def _make_copies(self):
+        """The unperturbed copies that model error fused into a step needs at
+        the block cadence, allocated once, outside any graph capture; the
+        marching kernel's model error has launches of its own and needs none."""
+        if getattr(self, "_noise", None) and self._noise_kind == "soar" and not self._marches():
+            _lib.call("goc_ensemble_set_block_noise", self._handle, self._noise, 0)
+            _lib.call("goc_ensemble_set_block_noise", self._handle, None, -1)
 
     def set_kl_random(self, member, normals):
         """Inject the (2 Ny, Nx) normals that member `member` (and every

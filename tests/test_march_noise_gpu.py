@@ -79,3 +79,29 @@ def test_blocks_without_steps_draw_nothing(gpu_ctx, shape, use_graph):
         out.append(_results(ens, sims))
         ens.release()
     assert _same(*out)
+
+
+def test_unperturbed_copies_where_a_step_needs_them(gpu_ctx):
+    """A marching engine allocates none of the copies that fused model error
+    reads; one that is given a tile shape later does, before its next block."""
+    import torch
+    from gpuocean_gb300.ensembles.BatchedEnsemble import BatchedEnsemble
+    out = []
+    for late in (False, True):
+        sims = [_member(gpu_ctx, 504, 301, (1, 2, 1, 2), 3 + m, drifters=20) for m in range(12)]
+        _with_noise(sims, 7, 1)
+        for s in sims:
+            s.updateDt()
+        ens = BatchedEnsemble(sims, autotune=False)
+        ens.set_tile_shape(ens.tile_shapes().index((56, 8) if late else (32, 16)))
+        free = torch.cuda.mem_get_info()[0]
+        ens.set_noise([s.model_error for s in sims], rng_seed=5)
+        used = free - torch.cuda.mem_get_info()[0]
+        copies = 12 * 3 * 4 * 508 * 305
+        assert used < copies if late else used >= copies
+        ens.step(120.0, True)
+        ens.set_tile_shape(0)
+        ens.step(120.0, True)
+        out.append(_results(ens, sims))
+        ens.release()
+    assert _same(*out)
