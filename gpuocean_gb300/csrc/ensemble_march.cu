@@ -9,12 +9,13 @@ constexpr int kMarchBlocks = 8;               // strips per SM: 128 registers a 
 
 // Work items: runs (member, strip, first unit, units) of kMarchRows rows, then
 // the drifter chunks of step k-1 (see ensemble_rk2_kernel); each CTA takes
-// item blockIdx.x first and every further one from the counter.
+// item blockIdx.x first and every further one from the counter.  const_f: every
+// member has one Coriolis value, and a table beside it counts for nothing.
 template <bool UNI>
 __global__ void __launch_bounds__(kMarchThreads, kMarchBlocks)
 ensemble_march_kernel(const GocCdklmParams pu, const StepConst ku, const MarchConst mu,
-                      const GocMemberDesc* __restrict__ members, const int4* __restrict__ runs, int n_runs,
-                      const float* __restrict__ dt_table, const int* __restrict__ nsub, int max_sub, int k,
+                      const GocMemberDesc* __restrict__ members, bool const_f, const int4* __restrict__ runs,
+                      int n_runs, const float* __restrict__ dt_table, const int* __restrict__ nsub, int max_sub, int k,
                       float* const* __restrict__ drift_pos, const int4* __restrict__ drift_chunks, int n_chunks,
                       float sensitivity, float* const* __restrict__ spare, const int* __restrict__ noise_steps,
                       int* queue) {
@@ -47,8 +48,8 @@ ensemble_march_kernel(const GocCdklmParams pu, const StepConst ku, const MarchCo
             S.m.k = make_step_const(S.m.p);
             S.m.c = make_march_const(S.m.p, S.m.k);
             S.grid = MarchGrid{d.eta[in], d.hu[in], d.hv[in], d.eta[out], d.hu[out], d.hv[out], nullptr, nullptr,
-                               nullptr, d.Hi, d.Hm, d.p.coriolis_cell, d.pitch / 4, d.Hi_pitch / 4, d.Hm_pitch / 4,
-                               d.p.coriolis_cell_pitch / 4};
+                               nullptr, d.Hi, d.Hm, const_f ? nullptr : d.p.coriolis_cell, d.pitch / 4,
+                               d.Hi_pitch / 4, d.Hm_pitch / 4, d.p.coriolis_cell_pitch / 4};
         }
         __syncthreads();
         const GocCdklmParams& ps = UNI ? pu : S.m.p;
@@ -90,8 +91,8 @@ static int march_launch_variant(Ensemble* e, int k, cudaStream_t st, const Fused
     const cudaError_t qe = cudaMemsetAsync(e->d_queue, 0, sizeof(int), st);
     if (qe != cudaSuccess) return set_error(GOC_ERR_CUDA, "ensemble work counter: %s", cudaGetErrorString(qe));
     ensemble_march_kernel<UNI><<<std::min(items, full), kMarchThreads, 0, st>>>(
-        e->pu, e->ku, make_march_const(e->pu, e->ku), e->d_members, e->d_march, e->n_march, e->d_dt, e->d_nsub,
-        e->max_substeps, k, e->d_drift_pos, e->d_step_chunks, e->n_step_chunks, e->drift_sensitivity,
+        e->pu, e->ku, make_march_const(e->pu, e->ku), e->d_members, e->const_f, e->d_march, e->n_march, e->d_dt,
+        e->d_nsub, e->max_substeps, k, e->d_drift_pos, e->d_step_chunks, e->n_step_chunks, e->drift_sensitivity,
         fn ? fn->spare : nullptr, e->d_nsub_noise, e->d_queue);
     count_launch();
     return check_launch("ensemble_march_kernel");
