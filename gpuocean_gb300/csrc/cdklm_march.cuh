@@ -13,9 +13,12 @@
 //     every intermediate through shared memory between block barriers).
 //     Values of the neighbouring columns come from warp shuffles.
 //   * two warps share a strip: the first evaluates stage 1 and leaves Q* in
-//     a ring of four rows in shared memory, the second marches a row behind
-//     with stage 2.  Each holds one stage's registers; they meet at a
-//     barrier per row.
+//     a ring of four rows in shared memory, the second marches three rows
+//     behind with stage 2: row r of stage 1 completes row r - 2 of Q*, which is
+//     read after the next barrier.  Each warp holds one stage's registers; they
+//     meet at a barrier per row.  What both read is kept in rings of eight rows:
+//     stage 2's oldest row lies five below the row of stage 1, the row that is
+//     on its way two above it.
 //   * rows of the inputs arrive two rows ahead in shared-memory rings
 //     (cp.async), at column addresses that are fixed for a run, so periodic
 //     images and wall mirrors cost nothing per row.
@@ -29,12 +32,12 @@
 // rounding by rounding (a value that several faces or terms of the tile
 // kernel recompute is evaluated once here), so both give the same bits.
 //
-// Measured (256 members of 512 x 300, one step): 1.41 ms against 2.42 ms of
-// the tile kernel; 96 members 0.566 against 0.945 ms, 917 thread
+// Measured (256 members of 512 x 300, one step): 1.39 ms against 2.42 ms of
+// the tile kernel; 96 members 0.566 against 0.945 ms, some 920 thread
 // instructions per cell (warp instructions x 32) against 1,910, 62 % of the
 // issue slots and 48 % of the FP32 pipe in use.  Eight strips per SM at 128
 // registers a thread; six at 168 (1.72 ms) leave too few warps, ten at 96
-// (1.75 ms) spill.
+// (1.75 ms) spill (128: none).
 #pragma once
 
 #include "cdklm_tile.cuh"
@@ -51,7 +54,6 @@ constexpr int kMarchThreads = 64;             // one warp per stage
 struct MarchGrid {
     const float* e; const float* hu; const float* hv;     // Q^n
     float* e_out; float* hu_out; float* hv_out;           // Q^{n+1}
-    float* e_star; float* hu_star; float* hv_star;        // first-stage state, or null
     const float* Hi; const float* Hm; const float* F;     // corner depths, cell means, Coriolis (or null)
     int pitch, hi_pitch, hm_pitch, f_pitch;               // floats
 };
@@ -805,12 +807,6 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
                 }
             } else {
                 const unsigned t4 = march_stage(r - 2);
-                if (__builtin_expect(G.e_star != nullptr, 0)) {
-                    if (r - 2 >= row0 && r - 2 < row1) {
-                        if (o0) { G.e_star[og] = qe.x; G.hu_star[og] = qu.x; G.hv_star[og] = qv.x; }
-                        if (o1) { G.e_star[og + 1] = qe.y; G.hu_star[og + 1] = qu.y; G.hv_star[og + 1] = qv.y; }
-                    }
-                }
                 at(ST, t4) = qe;
                 at(ST + P, t4) = qu;
                 at(ST + 2 * P, t4) = qv;

@@ -47,9 +47,9 @@ ensemble_march_kernel(const GocCdklmParams pu, const StepConst ku, const MarchCo
             S.m.p = d.p;
             S.m.k = make_step_const(S.m.p);
             S.m.c = make_march_const(S.m.p, S.m.k);
-            S.grid = MarchGrid{d.eta[in], d.hu[in], d.hv[in], d.eta[out], d.hu[out], d.hv[out], nullptr, nullptr,
-                               nullptr, d.Hi, d.Hm, const_f ? nullptr : d.p.coriolis_cell, d.pitch / 4,
-                               d.Hi_pitch / 4, d.Hm_pitch / 4, d.p.coriolis_cell_pitch / 4};
+            S.grid = MarchGrid{d.eta[in], d.hu[in], d.hv[in], d.eta[out], d.hu[out], d.hv[out], d.Hi, d.Hm,
+                               const_f ? nullptr : d.p.coriolis_cell, d.pitch / 4, d.Hi_pitch / 4, d.Hm_pitch / 4,
+                               d.p.coriolis_cell_pitch / 4};
         }
         __syncthreads();
         const GocCdklmParams& ps = UNI ? pu : S.m.p;
