@@ -166,6 +166,7 @@ class StepAdjoint:
             lib = _lib.load()
             b = self._bound_args = {
                 "step": lib.goc_cdklm_rk2_step, "stage": lib.goc_cdklm_rk2_step_stage,
+                "beside": lib.goc_cdklm_rk2_step_stage_beside,
                 "vjp": lib.goc_cdklm_stage_vjp_out,
                 "pre": (ctypes.byref(self.params), ctypes.c_float(self.dt)),
                 "common": (self.pitch, self.Hi.ptr, int(self.Hi.pitch), self.Hm.ptr, int(self.Hm.pitch)),
@@ -177,9 +178,9 @@ class StepAdjoint:
         b = self._bound()
         _lib.check(b["step"](*b["pre"], *src, *dst, *b["common"], stream), "goc_cdklm_rk2_step")
 
-    def _stage_p(self, src, dst, star, stream):
+    def _stage_p(self, src, dst, star, stream, entry="stage"):
         b = self._bound()
-        _lib.check(b["stage"](*b["pre"], *src, *dst, *star, *b["common"], stream), "goc_cdklm_rk2_step_stage")
+        _lib.check(b[entry](*b["pre"], *src, *dst, *star, *b["common"], stream), "goc_cdklm_rk2_step_stage")
 
     def _vjp_p(self, qn, qs, qnext, lam_next, lam_star, lam_n, stream):
         """step_vjp on addresses (q_next given)."""
@@ -318,7 +319,7 @@ def _rollout_backward(ctx, grad, grad_pos):
                 st[0].copy_(ckpt[start // K])
             bs, bt = st.data_ptr(), sr.data_ptr()
             for i in range(min(start + K, n_steps) - start):
-                adj._stage_p(_triple(bs, i, plane), _triple(bs, i + 1, plane), _triple(bt, i, plane), sh)
+                adj._stage_p(_triple(bs, i, plane), _triple(bs, i + 1, plane), _triple(bt, i, plane), sh, "beside")
             ready[b].record(side)
 
         recompute(order[0], 0)

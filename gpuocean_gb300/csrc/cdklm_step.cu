@@ -92,7 +92,7 @@ template <int NSTAGE>
 static int dispatch(const GocCdklmParams* p, const StepConst& k, bool cf, bool sf, float dt, int rk_step,
                     const float* e0, const float* hu0, const float* hv0, float* e1, float* hu1, float* hv1,
                     float* ea, float* hua, float* hva, int pitch_f, const float* Hi, int hi_pitch_f,
-                    const float* Hm, int hm_pitch_f, cudaStream_t st) {
+                    const float* Hm, int hm_pitch_f, cudaStream_t st, bool beside = false) {
     if constexpr (NSTAGE == 2) {
         // A step of a grid that leaves SMs idle, or one CTA on each, lasts as
         // long as one CTA does: with 256 threads 14.5 us from 64 x 64 to 256 x
@@ -103,10 +103,17 @@ static int dispatch(const GocCdklmParams* p, const StepConst& k, bool cf, bool s
         // step.  With two CTAs on an SM (512 x 300) the larger CTAs gain 2 us
         // alone and lose 1 of 10 us with others, so those keep 256 threads.
         const long long tiles = (long long)((p->nx + kTX - 1) / kTX) * ((p->ny + kTY - 1) / kTY);
-        if (sf && tiles <= kSMs / 4)
+        // Beside other kernels (the reverse sweep that a recomputed segment runs
+        // along with) such CTAs pay while they leave half of the SMs alone, and
+        // hold those kernels up when they do not: backward of 400 checkpointed
+        // steps, ms with them / with 256 threads: 64 x 64 11.6 / 11.8, 96 x 96
+        // 12.2 / 12.2, 128 x 128 12.7 / 12.4, 192 x 192 13.0 / 13.6, 224 x 224
+        // 15.1 / 14.4, 256 x 256 15.3 / 15.2.
+        const bool small = tiles <= kSMs / 4, alone = !beside || (small ? 4 : 1) * tiles <= kSMs / 2;
+        if (sf && alone && small)
             return cf ? launch_tile<2, true, true, false, 16, 8, 384>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st)
                       : launch_tile<2, false, true, false, 16, 8, 384>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st);
-        if (sf && tiles <= kSMs)
+        if (sf && alone && tiles <= kSMs)
             return cf ? launch_tile<2, true, true, false, kTX, kTY, 1024>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st)
                       : launch_tile<2, false, true, false, kTX, kTY, 1024>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st);
         // Large grids: 32 x 32 tiles recompute 1.27 instead of 1.41 of stage 1,
@@ -195,24 +202,40 @@ extern "C" int goc_cdklm_rk2_steps(const GocCdklmParams* p, const float* dts, in
     return GOC_OK;
 }
 
-extern "C" int goc_cdklm_rk2_step_stage(const GocCdklmParams* p, float dt, const float* eta0, const float* hu0,
-                                        const float* hv0, float* eta1, float* hu1, float* hv1, float* eta_s,
-                                        float* hu_s, float* hv_s, int pitch, const float* Hi, int Hi_pitch,
-                                        const float* Hm, int Hm_pitch, void* stream) {
-    int rc = validate_params(p, "goc_cdklm_rk2_step_stage");
+static int step_stage(const char* who, bool beside, const GocCdklmParams* p, float dt, const float* eta0,
+                      const float* hu0, const float* hv0, float* eta1, float* hu1, float* hv1, float* eta_s,
+                      float* hu_s, float* hv_s, int pitch, const float* Hi, int Hi_pitch, const float* Hm,
+                      int Hm_pitch, void* stream) {
+    int rc = validate_params(p, who);
     if (rc) return rc;
-    if ((rc = check_pitch(p, pitch, Hi_pitch, Hm_pitch, "goc_cdklm_rk2_step_stage"))) return rc;
+    if ((rc = check_pitch(p, pitch, Hi_pitch, Hm_pitch, who))) return rc;
     if (!eta0 || !hu0 || !hv0 || !eta1 || !hu1 || !hv1 || !eta_s || !hu_s || !hv_s || !Hi || !Hm)
-        return set_error(GOC_ERR_ARG, "goc_cdklm_rk2_step_stage: null buffer");
+        return set_error(GOC_ERR_ARG, "%s: null buffer", who);
     if (eta0 == eta1 || eta_s == eta0 || eta_s == eta1)
-        return set_error(GOC_ERR_ARG, "goc_cdklm_rk2_step_stage: the three buffer sets must differ");
-    if (p->rk_order != 2) return set_error(GOC_ERR_ARG, "goc_cdklm_rk2_step_stage: params.rk_order must be 2");
+        return set_error(GOC_ERR_ARG, "%s: the three buffer sets must differ", who);
+    if (p->rk_order != 2) return set_error(GOC_ERR_ARG, "%s: params.rk_order must be 2", who);
     StepConst k;
     bool cf, sf;
     cudaStream_t st = as_stream(stream);
     if ((rc = make_const(p, &k, &cf, &sf))) return rc;
     return dispatch<2>(p, k, cf, sf, dt, 1, eta0, hu0, hv0, eta1, hu1, hv1, eta_s, hu_s, hv_s, pitch / 4, Hi,
-                       Hi_pitch / 4, Hm, Hm_pitch / 4, st);
+                       Hi_pitch / 4, Hm, Hm_pitch / 4, st, beside);
+}
+
+extern "C" int goc_cdklm_rk2_step_stage(const GocCdklmParams* p, float dt, const float* eta0, const float* hu0,
+                                        const float* hv0, float* eta1, float* hu1, float* hv1, float* eta_s,
+                                        float* hu_s, float* hv_s, int pitch, const float* Hi, int Hi_pitch,
+                                        const float* Hm, int Hm_pitch, void* stream) {
+    return step_stage("goc_cdklm_rk2_step_stage", false, p, dt, eta0, hu0, hv0, eta1, hu1, hv1, eta_s, hu_s, hv_s,
+                      pitch, Hi, Hi_pitch, Hm, Hm_pitch, stream);
+}
+
+extern "C" int goc_cdklm_rk2_step_stage_beside(const GocCdklmParams* p, float dt, const float* eta0, const float* hu0,
+                                               const float* hv0, float* eta1, float* hu1, float* hv1, float* eta_s,
+                                               float* hu_s, float* hv_s, int pitch, const float* Hi, int Hi_pitch,
+                                               const float* Hm, int Hm_pitch, void* stream) {
+    return step_stage("goc_cdklm_rk2_step_stage_beside", true, p, dt, eta0, hu0, hv0, eta1, hu1, hv1, eta_s, hu_s, hv_s,
+                      pitch, Hi, Hi_pitch, Hm, Hm_pitch, stream);
 }
 
 extern "C" int goc_cdklm_rk2_step_members(const GocCdklmParams* p, float dt, const float* eta0, const float* hu0,

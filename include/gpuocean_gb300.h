@@ -142,7 +142,9 @@ int goc_cdklm_rk2_steps(const GocCdklmParams* p, const float* dts, int n_steps, 
  * goc_cdklm_rk2_step that also writes the first-stage state Q* of the
  * interior cells to (eta_s, hu_s, hv_s): the same values goc_cdklm_stage
  * with rk_step 0 gives, at no extra launch.  For the adjoint's recompute of
- * a rollout segment (no counterpart in the reference).
+ * a rollout segment (no counterpart in the reference).  The _beside form is
+ * the same step for a launch that runs along with other kernels: it chooses
+ * its tiles so as to leave them room.
  */
 int goc_cdklm_rk2_step_stage(const GocCdklmParams* p, float dt,
                              const float* eta0, const float* hu0, const float* hv0,
@@ -150,6 +152,12 @@ int goc_cdklm_rk2_step_stage(const GocCdklmParams* p, float dt,
                              float* eta_s, float* hu_s, float* hv_s, int pitch,
                              const float* Hi, int Hi_pitch, const float* Hm, int Hm_pitch,
                              void* stream);
+int goc_cdklm_rk2_step_stage_beside(const GocCdklmParams* p, float dt,
+                                    const float* eta0, const float* hu0, const float* hv0,
+                                    float* eta1, float* hu1, float* hv1,
+                                    float* eta_s, float* hu_s, float* hv_s, int pitch,
+                                    const float* Hi, int Hi_pitch, const float* Hm, int Hm_pitch,
+                                    void* stream);
 
 /*
  * One Runge-Kutta stage, reference semantics: cdklm_swe_2D
