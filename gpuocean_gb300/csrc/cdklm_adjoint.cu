@@ -604,13 +604,8 @@ static int dispatch_vjp(bool cf, bool hy, bool small, F&& f) {
 // 0.6 of the work (a launch of a few CTAs per SM is bound by one CTA's
 // latency, not by throughput).
 static bool small_tiles(const GocCdklmParams* p, int n_members) {
-    static int sms[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int& n = sms[dev & 63];
-    if (n == 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 0;
     const long long tiles = (long long)((p->nx + kAX - 1) / kAX) * ((p->ny + kAY - 1) / kAY) * n_members;
-    return n > 0 && tiles < 2LL * n;
+    return tiles < 2LL * sm_count();
 }
 
 // Wind partials: one (x, y) pair per tile of the smaller tile height, so the

@@ -86,8 +86,6 @@ static int launch_tile(const GocCdklmParams* p, const StepConst& k, float dt, in
     return check_launch("cdklm_tile_kernel");
 }
 
-constexpr int kSMs = 152;   // of a GB300
-
 template <int NSTAGE>
 static int dispatch(const GocCdklmParams* p, const StepConst& k, bool cf, bool sf, float dt, int rk_step,
                     const float* e0, const float* hu0, const float* hv0, float* e1, float* hu1, float* hv1,
@@ -102,6 +100,7 @@ static int dispatch(const GocCdklmParams* p, const StepConst& k, bool cf, bool s
         // Three simulators at once: 5.6 -> 4.0, 6.2 -> 4.6 and 6.6 -> 6.0 us a
         // step.  With two CTAs on an SM (512 x 300) the larger CTAs gain 2 us
         // alone and lose 1 of 10 us with others, so those keep 256 threads.
+        const int sms = sm_count();
         const long long tiles = (long long)((p->nx + kTX - 1) / kTX) * ((p->ny + kTY - 1) / kTY);
         // Beside other kernels (the reverse sweep that a recomputed segment runs
         // along with) such CTAs pay while they leave half of the SMs alone, and
@@ -109,11 +108,11 @@ static int dispatch(const GocCdklmParams* p, const StepConst& k, bool cf, bool s
         // steps, ms with them / with 256 threads: 64 x 64 11.6 / 11.8, 96 x 96
         // 12.2 / 12.2, 128 x 128 12.7 / 12.4, 192 x 192 13.0 / 13.6, 224 x 224
         // 15.1 / 14.4, 256 x 256 15.3 / 15.2.
-        const bool small = tiles <= kSMs / 4, alone = !beside || (small ? 4 : 1) * tiles <= kSMs / 2;
+        const bool small = tiles <= sms / 4, alone = !beside || (small ? 4 : 1) * tiles <= sms / 2;
         if (sf && alone && small)
             return cf ? launch_tile<2, true, true, false, 16, 8, 384>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st)
                       : launch_tile<2, false, true, false, 16, 8, 384>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st);
-        if (sf && alone && tiles <= kSMs)
+        if (sf && alone && tiles <= sms)
             return cf ? launch_tile<2, true, true, false, kTX, kTY, 1024>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st)
                       : launch_tile<2, false, true, false, kTX, kTY, 1024>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st);
         // Large grids: 32 x 32 tiles recompute 1.27 instead of 1.41 of stage 1,
@@ -121,7 +120,7 @@ static int dispatch(const GocCdklmParams* p, const StepConst& k, bool cf, bool s
         // 1501 x 1103 106.9 -> 101.8 us a step, three at once 100.6 -> 93.6;
         // 2400 x 1600 244 -> 228.  Below three waves of them the last, partly
         // empty one costs what they gain (1100 x 704, 2.5 waves: 57.6 -> 59.6).
-        if (sf && (long long)((p->nx + 31) / 32) * ((p->ny + 31) / 32) >= 6 * kSMs)
+        if (sf && (long long)((p->nx + 31) / 32) * ((p->ny + 31) / 32) >= 6 * sms)
             return cf ? launch_tile<2, true, true, false, 32, 32, 512>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st)
                       : launch_tile<2, false, true, false, 32, 32, 512>(p, k, dt, rk_step, e0, hu0, hv0, e1, hu1, hv1, ea, hua, hva, pitch_f, Hi, hi_pitch_f, Hm, hm_pitch_f, st);
     }

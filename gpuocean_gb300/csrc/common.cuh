@@ -21,6 +21,8 @@ constexpr float kMaxDt = 100000.0f;
 int set_error(int code, const char* fmt, ...);
 int check_launch(const char* what);
 void count_launch(int n = 1);
+// SMs of the current device (152 on a GB300).
+int sm_count();
 
 // Member tables of an ensemble handle (ensemble.cu): the descriptors as
 // created (host) and the device copy whose buffer set 0 is the current state.

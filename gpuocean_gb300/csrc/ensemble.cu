@@ -351,11 +351,9 @@ static int build_march(Ensemble* e) {
     cudaFree(e->d_march);
     e->d_march = nullptr;
     e->n_march = 0;
-    int grid = 0, dev = 0, sms = 1;
+    int grid = 0;
     const int rc = ensemble_march_configure(e, &grid);
     if (rc) return rc;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const TileShape sh = kEnsembleShapes[kMarchShape];
     long long units = 0, strips = 0;
     for (const GocMemberDesc& d : e->host) {
@@ -376,7 +374,7 @@ static int build_march(Ensemble* e) {
                                  std::min(strips, (long long)(tail * 0.5 * grid * most / per_strip))};
             if (tail && (most == 1 || plan.tail == 0)) continue;
             std::vector<int4> runs = march_runs(e, plan, strips);
-            const double t = march_makespan(runs, grid, std::max(1, grid / sms));
+            const double t = march_makespan(runs, grid, std::max(1, grid / sm_count()));
             if (best.empty() || t < best_t) {
                 best.swap(runs);
                 best_t = t;

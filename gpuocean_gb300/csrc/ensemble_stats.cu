@@ -268,7 +268,7 @@ __global__ void moments_finish_kernel(const GocMemberDesc* __restrict__ mem, int
 // members of 512 x 300, velocities: 39 us in one slice, 46 in two, 49 in three).
 static int moment_slices(int nx, int ny, int n, int* per_slice) {
     const long long blocks = (long long)((nx + 2 * kMX - 1) / (2 * kMX)) * ((ny + kMY - 1) / kMY);
-    const int most = (int)std::min<long long>(std::max<long long>(1, (152LL * kMBlocks + blocks - 1) / blocks),
+    const int most = (int)std::min<long long>(std::max<long long>(1, ((long long)sm_count() * kMBlocks + blocks - 1) / blocks),
                                               std::max(1, n / 16));
     *per_slice = (n + std::min(most, 65535) - 1) / std::min(most, 65535);
     return (n + *per_slice - 1) / *per_slice;
@@ -285,7 +285,7 @@ cudaError_t MomentScratch::create(const GocMemberDesc* members, int n_members) {
     for (int m = 0; m < n_members; ++m) {
         const GocCdklmParams& p = members[m].p;
         const long long blocks = (long long)((p.nx + 2 * kMX - 1) / (2 * kMX)) * ((p.ny + kMY - 1) / kMY);
-        const long long most = std::min<long long>((152LL * kMBlocks + blocks - 1) / blocks, n_members / 16);
+        const long long most = std::min<long long>(((long long)sm_count() * kMBlocks + blocks - 1) / blocks, n_members / 16);
         if (most > 1) floats = std::max(floats, (size_t)most * 6 * p.nx * p.ny);
     }
     if (floats == 0) return cudaSuccess;

@@ -32,6 +32,19 @@ int check_launch(const char* what) {
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
+int sm_count() {
+    static std::atomic<int> counts[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
+    std::atomic<int>& kept = counts[dev & 63];
+    int n = kept.load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+        kept.store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 static int cuda_result(cudaError_t e, const char* what) {
     if (e != cudaSuccess) return set_error(GOC_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
     return GOC_OK;
