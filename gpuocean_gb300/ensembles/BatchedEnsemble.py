@@ -15,7 +15,6 @@ different numbers of steps; a member whose block is done idles.
 from __future__ import annotations
 
 import ctypes
-import operator
 import threading
 
 import numpy as np
@@ -28,8 +27,6 @@ from ..utils import Common
 _AUTOTUNE_CACHE = {}
 # the tile shape that stands for the marching kernel
 MARCH_SHAPE = (56, 8)
-# a simulator's current state buffer, by which the engine sees that members were swapped or replaced
-_state_address = operator.attrgetter("gpu_data.h0.data.ptr")
 
 
 class _MomentBuffers:
@@ -227,7 +224,9 @@ class BatchedEnsemble:
         return descs
 
     def _current_ptrs(self):
-        return tuple(map(_state_address, self.sims))
+        """The members' current state buffers, by which the engine sees that
+        members were swapped or replaced."""
+        return [s.gpu_data.h0.data.ptr for s in self.sims]
 
     def _build(self, max_substeps=8):
         self._release_handles()
