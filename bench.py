@@ -42,10 +42,9 @@ NOISE_STD = 0.003         # target std of the SOAR eta perturbation [m]
 # by its member-cells.
 C3_SAMPLE = 96 * 512 * 300
 NCU_KERNELS = {
-    "ensemble_march_kernel": {"dram_bytes": 340.0e6 / C3_SAMPLE, "warp_inst": 0.4227e9 / C3_SAMPLE},
+    "ensemble_march_kernel": {"dram_bytes": 337.2e6 / C3_SAMPLE, "warp_inst": 0.4226e9 / C3_SAMPLE},
     "ensemble_rk2_kernel": {"dram_bytes": 369.7e6 / C3_SAMPLE, "warp_inst": 0.880e9 / C3_SAMPLE},
 }
-MARCH_SHAPE = (56, 8)
 SM_COUNT = 152
 
 
@@ -884,7 +883,7 @@ def main():
         ens._ptrs = ens._current_ptrs()
     ens._sched_key = None
     avg_bytes = float(np.mean(bytes_k))
-    kernel = "ensemble_march_kernel" if tuple(ens.tile_shape) == MARCH_SHAPE else "ensemble_rk2_kernel"
+    kernel = "ensemble_march_kernel" if ens._marches() else "ensemble_rk2_kernel"
     traffic = NCU_KERNELS[kernel]["dram_bytes"] * float(np.mean(cells_k))
     avg_dur = float(np.mean(durations))
     achieved = avg_bytes / avg_dur / 1e9
