@@ -636,7 +636,10 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
         // h + 0 (hu^2 + hv^2): NaN where a momentum is not finite, or so large that
         // a velocity might not be
         const float2 hf = fma2(fma2(hu, hu, mul2(hv, hv)), pr(0.0f), h);
-        bool bad = lands || !(min_nan(hf.x, hf.y) >= p.desing_eps);
+        // eta of a wet cell at the value that marks dry ones, which the scheme
+        // takes for one
+        const bool flag = eU.x == kDryFlag || eU.y == kDryFlag;
+        bool bad = lands || flag || !(min_nan(hf.x, hf.y) >= p.desing_eps);
 
         // ---- balanced x slope of row L and its depth check ----
         float2 wE, xE;
@@ -668,9 +671,9 @@ __device__ __forceinline__ void march_run(const GocCdklmParams& p, const GocCdkl
             bad = bad || bad_x;
         }
         bool slow = any_lane(bad);
-        // a row with land or a momentum that is not finite takes the general
-        // path until it has left the pipeline
-        if (__builtin_expect(slow, 0) && any_lane(lands || hf.x != hf.x || hf.y != hf.y)) hist |= 1u;
+        // a row with land, such a value or a momentum that is not finite takes
+        // the general path until it has left the pipeline
+        if (__builtin_expect(slow, 0) && any_lane(lands || flag || hf.x != hf.x || hf.y != hf.y)) hist |= 1u;
         if (!second) {
             // the depths that row U completes
             float2 A = at(CO, s4);

@@ -15,6 +15,8 @@ SPOTS = {
     "nan_momentum": [(1, 9, 20, np.nan)],
     "infinite_momentum": [(2, 12, 7, np.inf), (1, 20, 40, -np.inf)],
     "nan_eta": [(0, 10, 30, np.nan)],
+    # the value of eta that marks a dry cell, in wet ones
+    "dry_flag": [(0, 15, 30, 1e-30), (0, 16, 31, 1e-30), (0, 25, 4, 1e-30)],
     "huge": [(1, 14, 33, 1e25), (2, 5, 11, -1e30)],
     # rows at which a run of the queue starts, its pipeline rows, the domain's edges
     "many": [(q, j, i, v) for j in (2, 3, 7, 9, 10, 11, 17, 25) for q, i, v in
