@@ -121,39 +121,19 @@ __device__ __forceinline__ void pair_values(const float2* v, float eps, float2* 
 }
 
 // s += a with what the rounding lost kept in c (Kahan): the members' sums
-// would else run longer than those of a slice did.
-__device__ __forceinline__ void add_to(float2& s, float2& c, float2 a) {
-    const float2 y = make_float2(__fsub_rn(a.x, c.x), __fsub_rn(a.y, c.y));
-    const float2 t = make_float2(__fadd_rn(s.x, y.x), __fadd_rn(s.y, y.y));
-    c = make_float2(__fsub_rn(__fsub_rn(t.x, s.x), y.x), __fsub_rn(__fsub_rn(t.y, s.y), y.y));
+// would else run longer than those of a slice did.  A sum that is no longer
+// finite has lost nothing: inf - inf would make it NaN at the next member.
+// (Looking for such sums once, after the loop, and adding them up again without
+// compensation saves 1 % where there are none, but takes 316 instead of 67 us
+// where one of 96 members of 512 x 300 has blown up everywhere.)
+__device__ __forceinline__ void add_to(float& s, float& c, float a) {
+    const float y = __fsub_rn(a, c), t = __fadd_rn(s, y);
+    c = fabsf(t) < INFINITY ? __fsub_rn(__fsub_rn(t, s), y) : 0.0f;
     s = t;
 }
-
-struct CellSums { float s1[3], s2[3]; };
-
-// The sums of members [m0, m1) at one cell without compensation, which turns an
-// infinite sum to NaN at the next member: for the sums that are not finite in
-// the end.
-template <int Q>
-__device__ __noinline__ CellSums plain_sums(const GocMemberDesc* __restrict__ mem, int first, int m0, int m1, int x,
-                                            int y, float eps) {
-    constexpr int P = Q == 0 ? 3 : 2;
-    auto values = [&](int m, float* v) {
-        const GocMemberDesc& d = mem[m];
-        member_values<Q>(MomentSrc{d.eta[0], d.hu[0], d.hv[0], d.Hm, d.pitch / 4, d.Hm_pitch / 4}, x, y, eps, v);
-    };
-    CellSums sums{};
-    float K[P], v[P];
-    values(first, K);
-    for (int m = m0; m < m1; ++m) {
-        values(first + m, v);
-        for (int q = 0; q < P; ++q) {
-            const float e = v[q] - K[q];
-            sums.s1[q] += e;
-            sums.s2[q] += e * e;
-        }
-    }
-    return sums;
+__device__ __forceinline__ void add_to(float2& s, float2& c, float2 a) {
+    add_to(s.x, c.x, a.x);
+    add_to(s.y, c.y, a.y);
 }
 
 // One slice of the members: shifted sums s1 = sum(x - K), s2 = sum((x - K)^2)
@@ -166,7 +146,7 @@ __device__ __noinline__ CellSums plain_sums(const GocMemberDesc* __restrict__ me
 // thread, four members in flight and six slices took 92 us with their sum.  Four
 // blocks an SM leave 128 registers a thread: left to itself the compiler takes
 // 96 for the state, with fewer of the loads in flight (96 members 42.3 us instead
-// of 35.4, 256 members 93.7 instead of 77.4).
+// of 35.2, 256 members 93.7 instead of 76.4).
 template <int Q, bool WIDE>
 __global__ void __launch_bounds__(kMX * kMY, 4)
 moments_kernel(const GocMemberDesc* __restrict__ mem, int first, int n, int per_slice, int nx, int ny, int first_row,
@@ -246,19 +226,6 @@ moments_kernel(const GocMemberDesc* __restrict__ mem, int first, int n, int per_
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         if (x + h >= nx) break;
-        auto finite = [](float s) { return fabsf(s) < INFINITY; };
-        bool all = true;
-#pragma unroll
-        for (int q = 0; q < P; ++q) all = all && finite(h ? s1[q].y : s1[q].x) && finite(h ? s2[q].y : s2[q].x);
-        if (__builtin_expect(!all, 0)) {
-            const CellSums plain = plain_sums<Q>(mem, first, m0, m1, x + h, y, eps);
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-                float &a = h ? s1[q].y : s1[q].x, &b = h ? s2[q].y : s2[q].x;
-                if (!finite(a)) a = plain.s1[q];
-                if (!finite(b)) b = plain.s2[q];
-            }
-        }
         const size_t c = (size_t)y * nx + x + h;
 #pragma unroll
         for (int q = 0; q < P; ++q) {
